@@ -476,8 +476,10 @@ typedef struct SppTuneReport {
 } SppTuneReport;
 int spp_autotune(SppParams* p, const float* x, const float* y, const float* theta, int trial_steps,
                  int what, SppTuneReport* report);
-/* Number of kernels this handle has launched (graph replays count each
- * kernel node they run). */
+/* Number of kernels this handle has launched.  Graph replays count each
+ * kernel node they run; a resident run (many steps of a small or mid-sized
+ * Verlet-list system in one cooperative launch) counts the same stage and
+ * rebuild passes that a replay of its steps would have launched. */
 int64_t spp_kernel_launches(SppSystem* s);
 /* The cudaStream_t the handle launches on. */
 void* spp_stream(SppSystem* s);

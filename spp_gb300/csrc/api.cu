@@ -37,6 +37,7 @@ int fail(int status, const std::string& msg) {
   } while (0)
 
 constexpr int GRAPH_CHUNK = 32;
+constexpr int RUN_CHUNK = 1 << 14;   /* steps of one resident launch at most */
 
 struct GraphEntry {
   int nsteps;
@@ -77,6 +78,7 @@ struct SppSystem {
   bool uploaded = false;
   bool use_graphs = true;
   bool small_vicsek = false;     /* whole steps in one block (k_vicsek_small) */
+  RunPlan run = {0, 0, 0};          /* resident runs (k_run): launch shape, 0 blocks = the step graphs */
   float* stage_x = nullptr;      /* staging for uploads/downloads */
   float* stage_y = nullptr;
   float* stage_t = nullptr;
@@ -135,7 +137,7 @@ void free_dev(SppSystem* s) {
   DevState& d = s->d;
   void* ptrs[] = {d.pos, d.half, d.half2, d.theta, d.img, d.id, d.inv, d.kacc, d.dth, d.ref, d.pos_alt,
                   d.theta_alt, d.img_alt, d.id_alt, d.key, d.rank, d.cell_count, d.cell_start,
-                  d.scan_tmp, d.nbr, d.nn, d.long_q, d.nn_lanes, d.tumble, d.ctl, d.red, s->stage_x, s->stage_y, s->stage_t,
+                  d.scan_tmp, d.nbr, d.nn, d.long_q, d.nn_lanes, d.tumble, d.ctl, d.red, d.run_sums, s->stage_x, s->stage_y, s->stage_t,
                   s->stage_img};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -358,6 +360,18 @@ int run_steps(SppSystem* s, int64_t nsteps) {
     }
     return SPP_OK;
   }
+  if (s->run.blocks > 0) {
+    /* a stream that is being captured takes the graph path, which refuses it */
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CUDA_TRY(cudaStreamIsCapturing(s->stream, &cs));
+    while (cs == cudaStreamCaptureStatusNone && nsteps > 0) {
+      const int chunk = nsteps > RUN_CHUNK ? RUN_CHUNK : (int)nsteps;
+      if (launch_run(s->k, s->d, s->run, s->nstages, chunk, s->stream) != 0)
+        return fail(SPP_ERR_CUDA, std::string("k_run: ") + cudaGetErrorString(cudaGetLastError()));
+      s->graph_kernels += (int64_t)chunk * s->per_step_kernels;
+      nsteps -= chunk;
+    }
+  }
   while (nsteps > 0) {
     int chunk = nsteps >= GRAPH_CHUNK ? GRAPH_CHUNK : (int)nsteps;
     cudaGraphExec_t exec;
@@ -428,6 +442,9 @@ int recover(SppSystem* s) {
     Ctl c;
     int rc = read_ctl(s, &c);
     if (rc != SPP_OK) return rc;
+    if (c.run_timeout)
+      return fail(SPP_ERR_TIMEOUT, "a block of a resident run waited too long for the others; the state is not "
+                                   "reliable");
     if (c.bad_index)
       return fail(SPP_ERR_BOUNDS, "a kernel met an index out of range and skipped the access "
                                   "(SPP_CHECKED build); the state is not reliable");
@@ -776,6 +793,7 @@ int spp_create(const SppParams* p, SppSystem** out) {
   if (s->k.lanes > 1) rc = rc ? rc : dalloc(&d.nn_lanes, n);
   rc = rc ? rc : dalloc(&d.ctl, 1);
   rc = rc ? rc : dalloc(&d.red, 4);
+  rc = rc ? rc : dalloc(&d.run_sums, s->uses_list ? RUN_MAX_BLOCKS : 1);
   rc = rc ? rc : dalloc(&s->stage_x, n);
   rc = rc ? rc : dalloc(&s->stage_y, n);
   rc = rc ? rc : dalloc(&s->stage_t, n);
@@ -795,6 +813,10 @@ int spp_create(const SppParams* p, SppSystem** out) {
     return fail(SPP_ERR_CUDA, std::string("stream/ctl setup: ") + cudaGetErrorString(e));
   }
   s->own_stream = true;
+  {
+    const char* rv = getenv("SPP_RESIDENT");
+    if (s->uses_list && !(rv && rv[0] == '0')) plan_run(s->k, d, &s->run);
+  }
   s->per_rebuild_kernels = 7;   /* bin_count, scan x3, scatter, build_list, sort_long */
   s->per_step_kernels = s->uses_list ? (s->nstages == 1 ? 2 : s->nstages) : 6;
   *out = s;

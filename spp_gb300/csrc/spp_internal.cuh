@@ -42,6 +42,15 @@ struct Ctl {
   uint32_t long_n;        /* lists longer than the in-block sort queued by the last build */
   uint32_t bad_index;     /* SPP_CHECKED builds: a kernel met an index out of range */
   uint32_t bulk_timeouts; /* warps whose bulk copy of list rows did not arrive in time (they read global memory) */
+  /* resident runs (kernels_run.cu): largest squared displacements of step t
+   * in slot t % 3, blocks that have left the launch, a barrier wait that
+   * gave up, and the barrier's arrival count on a cache line of its own */
+  uint32_t run_disp[3], run_step[3];
+  uint32_t run_exit;
+  uint32_t run_timeout;
+  uint32_t pad0[32];
+  uint32_t run_bar;
+  uint32_t pad1[31];
 };
 
 /* SPP_CHECKED builds check every list, cell and slot index a hot kernel
@@ -90,6 +99,7 @@ struct DevState {
   int32_t* tumble;        /* run-and-tumble state by particle id (SPP_NOISE_TUMBLE), else NULL */
   Ctl* ctl;
   double* red;            /* reduction scratch (polarization) */
+  uint32_t* run_sums;     /* per-block cell totals of a resident run's rebuild (RUN_MAX_BLOCKS) */
 };
 
 /* api.cu: the device state, constants and stream of an uploaded system
@@ -135,6 +145,16 @@ void prepare_abp_stage();
 void launch_abp_stage(const SppConsts& k, const DevState& d, int stage, int nstages,
                       cudaGraphConditionalHandle cond, int use_cond, cudaStream_t s,
                       int64_t* launches);
+/* kernels_run.cu: nsteps whole steps of a Verlet-list system in one
+ * cooperative launch.  plan_run: whether the system fits (every thread of
+ * its neighbour sums resident at once) and the launch shape. */
+#define RUN_MAX_BLOCKS 1024
+struct RunPlan {
+  int blocks, threads;    /* 0: the system does not fit */
+  int per_sm;             /* blocks per SM the kernel is compiled for (1 or 2) */
+};
+bool plan_run(const SppConsts& k, const DevState& d, RunPlan* plan);
+int launch_run(const SppConsts& k, const DevState& d, const RunPlan& plan, int nstages, int nsteps, cudaStream_t s);
 void launch_vicsek_step(const SppConsts& k, const DevState& d, cudaStream_t s, int64_t* launches);
 /* Whole Vicsek steps of a small system in one thread-block cluster
  * (k_vicsek_small): at most SPP_SMALL_MAX_N particles, fewer than 65536
