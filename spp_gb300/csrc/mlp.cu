@@ -18,6 +18,7 @@
  * atomics, hence reproducible), Adam elementwise.
  */
 #include <cuda_bf16.h>
+#include <cooperative_groups.h>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -552,21 +553,26 @@ __global__ void k_mlp_loss(MlpDev m, float* loss) {
 /* Adam (Kingma & Ba, 2015) on the FP32 masters; refreshes the BF16 copy.
  * The bias corrections of step t are bias[*tix] = (1 - b1^t, 1 - b2^t),
  * tabulated on the host for the steps of one training call. */
+struct AdamState { float th, mom, vel; };
+__device__ __forceinline__ void adam_step(AdamState* a, float g, float2 c, float lr, float b1, float b2, float eps) {
+  const float mm = b1 * a->mom + (1.0f - b1) * g;
+  const float vv = b2 * a->vel + (1.0f - b2) * g * g;
+  a->mom = mm;
+  a->vel = vv;
+  a->th = a->th - lr * (mm / c.x) / (sqrtf(vv / c.y) + eps);
+}
+
 __global__ void k_mlp_adam(int count, float* master, __nv_bfloat16* w, const float* grad, float* mom,
                            float* vel, float lr, float b1, float b2, float eps, const float2* bias,
                            const int* tix) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  const float2 c = bias[*tix];
-  const float c1 = c.x, c2 = c.y;
-  const float g = grad[i];
-  const float mm = b1 * mom[i] + (1.0f - b1) * g;
-  const float vv = b2 * vel[i] + (1.0f - b2) * g * g;
-  mom[i] = mm;
-  vel[i] = vv;
-  const float th = master[i] - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
-  master[i] = th;
-  w[i] = __float2bfloat16_rn(th);
+  AdamState a = {master[i], mom[i], vel[i]};
+  adam_step(&a, grad[i], bias[*tix], lr, b1, b2, eps);
+  mom[i] = a.mom;
+  vel[i] = a.vel;
+  master[i] = a.th;
+  w[i] = __float2bfloat16_rn(a.th);
 }
 
 __global__ void k_mlp_next(int* tix) { *tix += 1; }
@@ -574,6 +580,465 @@ __global__ void k_mlp_next(int* tix) { *tix += 1; }
 __global__ void k_mlp_cast(int count, const float* master, __nv_bfloat16* w) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) w[i] = __float2bfloat16_rn(master[i]);
+}
+
+/* ------------------------------------------------------------------ */
+/* whole training runs: one thread-block cluster per ensemble member     */
+/* ------------------------------------------------------------------ */
+/* k_mlp_train runs every iteration of a training call in one launch.  The
+ * members are independent, so each is one cluster of 16 CTAs, and the only
+ * synchronisation is two hardware cluster barriers per iteration:
+ *   A  the CTAs share the tiles of 16 samples, two at a time (eight warps
+ *      each): forward pass and per-sample deltas, the steps of
+ *      k_mlp_fused<true>, gelu and its derivative from one evaluation;
+ *   B  the CTAs share the parameters, the samples' activations and deltas
+ *      staged in shared memory by asynchronous copies: eight warps take one
+ *      of the 16 tiles of 32 x 32 of W2 (the products of k_mlp_grads_tc, a
+ *      warp per 16 x 8 entries), the other eight the remaining parameters of
+ *      8 hidden units (the sums of k_mlp_grad_small); each parameter's Adam
+ *      step follows at once.  Masters and moments stay with their owners (W2
+ *      in registers, the others in shared memory) until the last iteration
+ *      writes them back; the BF16 weights the next iteration reads are
+ *      published through `pub` (16-byte aligned).
+ * Every sum keeps the order of the kernels named above, so the trained
+ * parameters are the same bits.
+ *
+ * Why: an iteration is 0.16 GFLOP in five dependent launches that leave the
+ * GPU empty (10% issue active, 6% of warp slots).  Measured (us per
+ * iteration, graphs of the five launches -> this): 5 members x 60 samples
+ * 35.9 -> 12.8, 5 x 300 55.4 -> 20.6, 5 x 1000 137 -> 49, 5 x 10,000 1338 ->
+ * 445, 16 x 512 102 -> 79, 32 x 3000 941 -> 663, so every batch takes it.
+ * At 5 x 300 an iteration is 38,000 cycles: the chain of 3 x 38 dependent
+ * mma.sync of a W2 entry (8,800: 77 each), the two 128 x 128 products (2,400
+ * each, 4,300 where a CTA has two tiles), staging 106 KB per CTA (4,700),
+ * weights (2,100), the first layer (2,000 to 3,200), gelu, the output sum,
+ * Adam and the two barriers (1,400 each).  Slower variants: W2 kept as BF16
+ * in shared memory and staging in four parts (24.6 at 5 x 300), staging in
+ * two parts (21.0), 256 threads (26.2). */
+constexpr int TR = 16;                  /* CTAs per cluster */
+constexpr int TT = 512;                 /* threads: two groups of eight warps */
+constexpr int TG = TT / 2;
+constexpr int TJ = H / TR;              /* hidden units per CTA in phase B */
+constexpr int TR_CH = 304;              /* samples staged at a time in phase B (a multiple of 8) */
+constexpr int TR_GP = 40;               /* row stride of the staged 32-column tiles: 8 t + g, all banks differ */
+/* published weights of a member: W2, W1, b1, b2, W3, b3 */
+__host__ __device__ inline int pub_size(int in) { return (n_params(in) + 7) / 8 * 8; }
+__host__ __device__ inline int pub_w1() { return H * H; }
+/* parameters outside W2 of one CTA: W1 rows, b1, b2, W3 of its units, and
+ * (the first CTA's) b3 */
+constexpr int TR_MAX_ITEMS = TJ * (MAX_IN + 3) + 1;
+constexpr int TR_ROUNDS = (TR_MAX_ITEMS + TG / GSPLIT - 1) / (TG / GSPLIT);
+/* floats of dynamic shared memory: phase A's W2 and its two groups' tiles {
+ * h1, h2 / dz2 [16][HP], gelu'(z1) [16][H], dy [16], x [16][in] }, phase B's staged
+ * samples { dz2, h1 [TR_GP], dz1, dz2, h2 [TJ], dy } in the same bytes;
+ * before them the small weights, their Adam states and the batch's inputs
+ * (up to TR_CH samples) */
+constexpr int TR_TILE = 2 * 16 * HP + 16 * H + 16 + 16 * MAX_IN;
+constexpr int TR_A = H * WP + 2 * TR_TILE;
+constexpr int TR_B = TR_CH * (2 * TR_GP + 3 * TJ + 1);
+__host__ __device__ inline int train_fixed_floats(int in) {
+  return (H * in + 3 * H + 8 + 3 * (TJ * (in + 3) + 1) + TR_CH * in + 3) / 4 * 4;
+}
+__host__ __device__ inline size_t train_smem_bytes(int in) {
+  return sizeof(float) * (size_t)(train_fixed_floats(in) + (TR_A > TR_B ? TR_A : TR_B));
+}
+
+struct TrainArgs {
+  MlpDev m;
+  float *master, *mom, *vel;            /* [E][P] */
+  __nv_bfloat16* w;                     /* [E][P] */
+  __nv_bfloat16* pub;                   /* [E][pub_size] */
+  const float2* bias;                   /* Adam bias corrections of the iterations */
+  int iters;
+  float lr, b1, b2, eps;
+};
+
+__device__ __forceinline__ void tile_sync(int group) {
+  if (group == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+  else asm volatile("bar.sync 2, 256;" ::: "memory");
+}
+static_assert(TG == 256, "tile_sync's thread count");
+
+/* 16 bytes from global (L2) to shared memory, asynchronously */
+__device__ __forceinline__ void copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+/* item u of the CTA that owns units j0 .. j0 + TJ - 1 -> parameter index
+ * (kind 0: W1, 1: b1, 2: b2, 3: W3, 4: b3) */
+__device__ __forceinline__ int train_item(int u, int in, int j0, int* kind, int* j, int* k) {
+  *k = 0;
+  if (u < TJ * in) {
+    *kind = 0;
+    *j = u / in;
+    *k = u % in;
+    return (j0 + *j) * in + *k;
+  }
+  u -= TJ * in;
+  if (u >= 3 * TJ) {
+    *kind = 4;
+    *j = 0;
+    return off_b3(in);
+  }
+  *kind = 1 + u / TJ;
+  *j = u % TJ;
+  return (*kind == 1 ? off_b1(in) : (*kind == 2 ? off_b2(in) : off_w3(in))) + j0 + *j;
+}
+
+/* acc[nt] += A B over the 128 rows of k for the 16 x 16 tile of columns
+ * n0 .. n0 + 15: A the FP32 tile `act` (split hi + lo), B the weights
+ * (row n of W2, or with TRANS column n) */
+template <bool TRANS>
+__device__ __forceinline__ void layer_mma(float (*acc)[4], const float* act, const float* w2f, int n0, int g, int t) {
+#pragma unroll 4
+  for (int k0 = 0; k0 < H; k0 += 8) {
+    uint32_t ah[4], al[4];
+    tf32_split(act[g * HP + k0 + t], &ah[0], &al[0]);
+    tf32_split(act[(g + 8) * HP + k0 + t], &ah[1], &al[1]);
+    tf32_split(act[g * HP + k0 + t + 4], &ah[2], &al[2]);
+    tf32_split(act[(g + 8) * HP + k0 + t + 4], &ah[3], &al[3]);
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+      const int n = n0 + nt * 8 + g;
+      const uint32_t b0 = __float_as_uint(TRANS ? w2f[(k0 + t) * WP + n] : w2f[n * WP + k0 + t]);
+      const uint32_t b1 = __float_as_uint(TRANS ? w2f[(k0 + t + 4) * WP + n] : w2f[n * WP + k0 + t + 4]);
+      mma_tf32(acc[nt], ah, b0, b1);
+      mma_tf32(acc[nt], al, b0, b1);
+    }
+  }
+}
+
+/* The sums of one small parameter over the staged samples s = r8, r8 + 8, ..
+ * below n, continued from gsum in that order. */
+__device__ __forceinline__ float unit_sum(float gsum, int kind, int r8, int n, const float* d, const float* x, int in) {
+  if (kind == 0) {         /* dz1 x */
+#pragma unroll 8
+    for (int s = r8; s < n; s += GSPLIT) gsum = fmaf(d[s * TJ], x[s * in], gsum);
+  } else if (kind == 3) {  /* dy h2 */
+#pragma unroll 8
+    for (int s = r8; s < n; s += GSPLIT) gsum = fmaf(x[s], d[s * TJ], gsum);
+  } else if (kind == 4) {
+#pragma unroll 8
+    for (int s = r8; s < n; s += GSPLIT) gsum += x[s];
+  } else {
+#pragma unroll 8
+    for (int s = r8; s < n; s += GSPLIT) gsum += d[s * TJ];
+  }
+  return gsum;
+}
+
+__global__ void __launch_bounds__(TT, 1) k_mlp_train(TrainArgs a) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ __align__(16) float tsm[];
+  const MlpDev& m = a.m;
+  const int rk = (int)cluster.block_rank();
+  const int e = blockIdx.x / TR;
+  const int in = m.in, P = n_params(in), B = m.B;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int group = warp >> 3, gw = warp & 7, gt = tid & (TG - 1);
+  const int ju = rk * TJ;                           /* this CTA's hidden units in phase B */
+  const int items = TJ * (in + 3) + (rk == 0 ? 1 : 0);
+  float* const w1s = tsm;                           /* [H][in] */
+  float* const b1s = w1s + H * in;
+  float* const b2s = b1s + H;
+  float* const w3s = b2s + H;
+  float* const b3s = w3s + H;                       /* 1 (padded to 8) */
+  AdamState* const st = reinterpret_cast<AdamState*>(b3s + 8);
+  float* const xs = reinterpret_cast<float*>(st + TJ * (in + 3) + 1);   /* [TR_CH][in] */
+  float* const work = tsm + train_fixed_floats(in);
+  const size_t eb = (size_t)e * B;
+  __nv_bfloat16* const pub = a.pub + (size_t)e * pub_size(in);
+  float* const master = a.master + (size_t)e * P;
+  float* const mom = a.mom + (size_t)e * P;
+  float* const vel = a.vel + (size_t)e * P;
+  __nv_bfloat16* const wout = a.w + (size_t)e * P;
+  const int tiles = (B + 15) / 16;
+
+  /* the W2 entries of a thread of the first eight warps */
+  const int j0 = (rk >> 2) * 32, k0 = (rk & 3) * 32;
+  const int wm = (warp >> 2) * 16, wn = (warp & 3) * 8;
+  auto w2_index = [&](int c) { return (j0 + wm + g + (c >= 2 ? 8 : 0)) * H + k0 + wn + 2 * t + (c & 1); };
+  AdamState own[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    own[c] = {0.0f, 0.0f, 0.0f};
+    if (group == 0) {
+      const int q = off_w2(in) + w2_index(c);
+      own[c] = {master[q], mom[q], vel[q]};
+    }
+  }
+  for (int u = tid; u < items; u += TT) {
+    int kind, j, k;
+    const int q = train_item(u, in, ju, &kind, &j, &k);
+    st[u] = {master[q], mom[q], vel[q]};
+  }
+
+  const bool x_here = B <= TR_CH;
+  if (x_here)
+    for (int idx = tid; idx < B * in; idx += TT) xs[idx] = __ldg(m.x + idx);
+  /* the small parameters of a thread of the last eight warps (eight threads
+   * each): place in the staged deltas, in the inputs, kind */
+  const int r8 = gt % GSPLIT, u8 = gt / GSPLIT;
+  int item_j[TR_ROUNDS], item_k[TR_ROUNDS], item_kind[TR_ROUNDS];
+#pragma unroll
+  for (int w = 0; w < TR_ROUNDS; ++w) {
+    const int u = w * (TG / GSPLIT) + u8;
+    item_kind[w] = -1;
+    item_j[w] = item_k[w] = 0;
+    if (u < items) train_item(u, in, ju, &item_kind[w], &item_j[w], &item_k[w]);
+  }
+
+  for (int it = 0; it < a.iters; ++it) {
+    /* ---- A: weights, then the tiles ---- */
+    float* const w2f = work;
+    constexpr int NW = H * H / 8 / TT, NS = (H * MAX_IN + 3 * H + 1 + TT - 1) / TT;
+    const int nsmall = H * in + 3 * H + 1;
+    uint4 wv[NW];
+    unsigned short sv[NS];
+#pragma unroll
+    for (int q = 0; q < NW; ++q) wv[q] = __ldcg(reinterpret_cast<const uint4*>(pub) + tid + q * TT);
+#pragma unroll
+    for (int q = 0; q < NS; ++q)
+      if (tid + q * TT < nsmall) sv[q] = __ldcg(reinterpret_cast<const unsigned short*>(pub) + pub_w1() + tid + q * TT);
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      const int idx = tid + w * TT;
+      const uint32_t u[4] = {wv[w].x, wv[w].y, wv[w].z, wv[w].w};
+      float* const dst = w2f + (idx * 8 / H) * WP + (idx * 8) % H;
+      float f[8];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {   /* BF16 bits are the upper half of the FP32 value */
+        f[2 * q] = __uint_as_float(u[q] << 16);
+        f[2 * q + 1] = __uint_as_float(u[q] & 0xffff0000u);
+      }
+      reinterpret_cast<float4*>(dst)[0] = make_float4(f[0], f[1], f[2], f[3]);
+      reinterpret_cast<float4*>(dst)[1] = make_float4(f[4], f[5], f[6], f[7]);
+    }
+#pragma unroll
+    for (int q = 0; q < NS; ++q)
+      if (tid + q * TT < nsmall) w1s[tid + q * TT] = __uint_as_float((uint32_t)sv[q] << 16);
+    __syncthreads();
+    float* const hs = work + H * WP + group * TR_TILE;         /* [16][HP]: h1 */
+    float* const t2 = hs + 16 * HP;                          /* [16][HP]: h2, then dz2 */
+    float* const g1s = t2 + 16 * HP;                         /* [16][H]: gelu'(z1) */
+    float* const dys = g1s + 16 * H;
+    float* const xtile = dys + 16;
+    for (int tile = rk + group * TR; tile < tiles; tile += 2 * TR) {
+      const int s0 = tile * 16;
+      const int nq = B - s0 < 16 ? B - s0 : 16;
+      const float* xt = xs + s0 * in;
+      if (!x_here) {
+        for (int idx = gt; idx < nq * in; idx += TG) xtile[idx] = __ldg(m.x + (size_t)s0 * in + idx);
+        xt = xtile;
+        tile_sync(group);
+      }
+      {
+        /* unit gt % 128, samples gt / 128, + 2, ..; rows past the batch
+         * repeat the last sample and are cleared */
+        const int j = gt & (H - 1), qh = gt >> 7;
+        float z[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) z[u] = b1s[j];
+        for (int k = 0; k < in; ++k) {
+          const float wk = w1s[j * in + k];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) z[u] = fmaf(wk, xt[min(2 * u + qh, nq - 1) * in + k], z[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int q = 2 * u + qh;
+          float dg;
+          const float h = gelu(z[u], &dg);
+          if (q < nq) m.h1[(eb + s0 + q) * H + j] = h;
+          hs[q * HP + j] = q < nq ? h : 0.0f;
+          g1s[q * H + j] = dg;
+        }
+      }
+      tile_sync(group);
+      float acc[2][4], g2[2][4];
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[nt][c] = 0.0f;
+      layer_mma<false>(acc, hs, w2f, gw * 16, g, t);
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int q = g + (c >= 2 ? 8 : 0);
+          const int j = gw * 16 + nt * 8 + 2 * t + (c & 1);
+          const float z2 = acc[nt][c] + b2s[j];
+          const float h2 = gelu(z2, &g2[nt][c]);
+          t2[q * HP + j] = q < nq ? h2 : 0.0f;
+          if (q < nq) m.h2[(eb + s0 + q) * H + j] = h2;
+        }
+      tile_sync(group);
+      if (gt < 16) {
+        float dy = 0.0f;
+        if (gt < nq) {
+          const size_t es = eb + s0 + gt;
+          const float sw = m.sw[es], ts = m.t[s0 + gt];
+          float yy = b3s[0];
+#pragma unroll 8
+          for (int j = 0; j < H; j += 4) {
+            const float4 hv = *reinterpret_cast<const float4*>(t2 + gt * HP + j);
+            const float4 w3 = *reinterpret_cast<const float4*>(w3s + j);
+            yy = fmaf(w3.x, hv.x, yy);
+            yy = fmaf(w3.y, hv.y, yy);
+            yy = fmaf(w3.z, hv.z, yy);
+            yy = fmaf(w3.w, hv.w, yy);
+          }
+          dy = 2.0f * sw * (yy - ts);
+          m.dy[es] = dy;
+        }
+        dys[gt] = dy;
+      }
+      tile_sync(group);
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int q = g + (c >= 2 ? 8 : 0);
+          const int j = gw * 16 + nt * 8 + 2 * t + (c & 1);
+          const float dz2 = dys[q] * w3s[j] * g2[nt][c];
+          t2[q * HP + j] = dz2;
+          if (q < nq) m.dz2[(eb + s0 + q) * H + j] = dz2;
+          acc[nt][c] = 0.0f;
+        }
+      tile_sync(group);
+      layer_mma<true>(acc, t2, w2f, gw * 16, g, t);
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int q = g + (c >= 2 ? 8 : 0);
+          const int k = gw * 16 + nt * 8 + 2 * t + (c & 1);
+          if (q < nq) m.dz1[(eb + s0 + q) * H + k] = acc[nt][c] * g1s[q * H + k];
+        }
+      tile_sync(group);   /* the group's tile buffers are free */
+    }
+    cluster.sync();       /* every tile's activations and deltas are written */
+
+    /* ---- B: gradients and Adam ---- */
+    const float2 corr = __ldg(a.bias + it);
+    const bool final = it == a.iters - 1;
+    float* const dzs = work;                 /* [TR_CH][TR_GP]: dz2[s][j0 + c] */
+    float* const h1t = dzs + TR_CH * TR_GP;  /* [TR_CH][TR_GP]: h1[s][k0 + c] */
+    float* const d1t = h1t + TR_CH * TR_GP;  /* [TR_CH][TJ]: dz1 */
+    float* const d2t = d1t + TR_CH * TJ;     /* [TR_CH][TJ]: dz2 */
+    float* const h2t = d2t + TR_CH * TJ;     /* [TR_CH][TJ]: h2 */
+    float* const dyt = h2t + TR_CH * TJ;     /* [TR_CH] */
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float gsum[TR_ROUNDS];
+#pragma unroll
+    for (int w = 0; w < TR_ROUNDS; ++w) gsum[w] = 0.0f;
+    for (int c0 = 0; c0 < B; c0 += TR_CH) {
+      const int nc = B - c0 < TR_CH ? B - c0 : TR_CH;
+      const int np = (nc + 7) & ~7;
+      if (c0 > 0) __syncthreads();   /* the chunk before is used up */
+      for (int idx = tid; idx < np * 8; idx += TT) {
+        const int r = idx >> 3, c = (idx & 7) * 4;
+        if (r < nc) {
+          copy16(dzs + r * TR_GP + c, m.dz2 + (eb + c0 + r) * H + j0 + c);
+          copy16(h1t + r * TR_GP + c, m.h1 + (eb + c0 + r) * H + k0 + c);
+        } else {
+          *reinterpret_cast<float4*>(dzs + r * TR_GP + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          *reinterpret_cast<float4*>(h1t + r * TR_GP + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+      }
+      for (int idx = tid; idx < nc * (TJ / 4); idx += TT) {
+        const int r = idx / (TJ / 4), c = (idx % (TJ / 4)) * 4;
+        const size_t es = (eb + c0 + r) * H + ju + c;
+        copy16(d1t + r * TJ + c, m.dz1 + es);
+        copy16(d2t + r * TJ + c, m.dz2 + es);
+        copy16(h2t + r * TJ + c, m.h2 + es);
+      }
+      for (int idx = tid; idx < nc; idx += TT) dyt[idx] = __ldcg(m.dy + eb + c0 + idx);
+      if (!x_here)      /* a batch of one chunk has its inputs there already */
+        for (int idx = tid; idx < nc * in; idx += TT) xs[idx] = __ldg(m.x + (size_t)c0 * in + idx);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      if (group == 0) {
+#pragma unroll 4
+        for (int s8 = 0; s8 < np; s8 += 8) {
+          uint32_t ah[4], al[4], bh0, bl0, bh1, bl1;
+          tf32_split(dzs[(s8 + t) * TR_GP + wm + g], &ah[0], &al[0]);
+          tf32_split(dzs[(s8 + t) * TR_GP + wm + g + 8], &ah[1], &al[1]);
+          tf32_split(dzs[(s8 + t + 4) * TR_GP + wm + g], &ah[2], &al[2]);
+          tf32_split(dzs[(s8 + t + 4) * TR_GP + wm + g + 8], &ah[3], &al[3]);
+          tf32_split(h1t[(s8 + t) * TR_GP + wn + g], &bh0, &bl0);
+          tf32_split(h1t[(s8 + t + 4) * TR_GP + wn + g], &bh1, &bl1);
+          mma_tf32(acc, ah, bh0, bh1);
+          mma_tf32(acc, ah, bl0, bl1);
+          mma_tf32(acc, al, bh0, bh1);
+        }
+      } else {
+        /* TR_CH is a multiple of 8: sample c0 + s belongs to thread s % 8 */
+#pragma unroll
+        for (int q = 0; q < TR_ROUNDS; ++q) {
+          const int kind = item_kind[q];
+          if (kind >= 0) {
+            const float* const d = (kind == 2 ? d2t : (kind == 3 ? h2t : d1t)) + item_j[q];
+            gsum[q] = unit_sum(gsum[q], kind, r8, nc, d, kind == 0 ? xs + item_k[q] : dyt, in);
+          }
+        }
+      }
+    }
+    if (group == 0) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) adam_step(&own[c], acc[c], corr, a.lr, a.b1, a.b2, a.eps);
+#pragma unroll
+      for (int c = 0; c < 4; c += 2)   /* an even index: the pair is one aligned word */
+        *reinterpret_cast<__nv_bfloat162*>(pub + w2_index(c)) =
+            __halves2bfloat162(__float2bfloat16_rn(own[c].th), __float2bfloat16_rn(own[c + 1].th));
+      if (final) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int q = off_w2(in) + w2_index(c);
+          master[q] = own[c].th;
+          mom[q] = own[c].mom;
+          vel[q] = own[c].vel;
+          wout[q] = __float2bfloat16_rn(own[c].th);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int w = 0; w < TR_ROUNDS; ++w) {
+        float s = gsum[w];
+#pragma unroll
+        for (int o = 1; o < GSPLIT; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const int u = w * (TG / GSPLIT) + u8;
+        if (u < items && r8 == 0) {
+          int kind, j, k;
+          const int q = train_item(u, in, ju, &kind, &j, &k);
+          AdamState s2 = st[u];
+          adam_step(&s2, s, corr, a.lr, a.b1, a.b2, a.eps);
+          st[u] = s2;
+          const __nv_bfloat16 low = __float2bfloat16_rn(s2.th);
+          pub[pub_w1() + (q < off_w2(in) ? q : q - H * H)] = low;
+          if (final) {
+            master[q] = s2.th;
+            mom[q] = s2.mom;
+            vel[q] = s2.vel;
+            wout[q] = low;
+          }
+        }
+      }
+    }
+    cluster.sync();       /* the next iteration's weights are published */
+  }
+}
+
+/* The published layout of the current BF16 weights. */
+__global__ void k_mlp_publish(int E, int in, const __nv_bfloat16* w, __nv_bfloat16* pub) {
+  const int P = n_params(in);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= E * P) return;
+  const int e = i / P, q = i % P;
+  const int to = q < off_w2(in) ? pub_w1() + q : (q < off_b2(in) ? q - off_w2(in) : pub_w1() + q - H * H);
+  pub[(size_t)e * pub_size(in) + to] = w[i];
 }
 
 int mfail(int status, const std::string& msg) {
@@ -611,6 +1076,8 @@ struct SppMlp {
    * SPP_MLP_SCALAR=1 at creation selects the scalar FP32 kernels */
   bool tensor_cores = true;
   std::vector<TrainGraph> graphs;
+  __nv_bfloat16* pub = nullptr;   /* weights as k_mlp_train reads them */
+  bool train_cluster = false;     /* k_mlp_train fits the device; else the iteration graphs */
 };
 
 namespace {
@@ -754,6 +1221,64 @@ int mlp_train_graph(SppMlp* m, int B, float lr, cudaGraphExec_t* out) {
   return SPP_OK;
 }
 
+/* Whether the device takes k_mlp_train's cluster of 16 CTAs at in_dim
+ * inputs. */
+bool train_cluster_fits(int in) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = TR;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(TR);
+  cfg.blockDim = dim3(TT);
+  cfg.dynamicSmemBytes = train_smem_bytes(in);
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  const bool fits =
+      cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+      cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)train_smem_bytes(MAX_IN)) == cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&n, k_mlp_train, &cfg) == cudaSuccess && n > 0;
+  cudaGetLastError();
+  return fits;
+}
+
+bool train_in_cluster(const SppMlp* m, int B) { return m->tensor_cores && m->train_cluster; }
+
+int mlp_train_cluster(SppMlp* m, int B, int iters, float lr) {
+  const int tot = m->E * m->P;
+  k_mlp_publish<<<(tot + 255) / 256, 256, 0, m->stream>>>(m->E, m->in, m->w, m->pub);
+  TrainArgs a;
+  a.m = mlp_dev(m, B);
+  a.master = m->master;
+  a.mom = m->mom;
+  a.vel = m->vel;
+  a.w = m->w;
+  a.pub = m->pub;
+  a.bias = m->bias;
+  a.iters = iters;
+  a.lr = lr;
+  a.b1 = ADAM_B1;
+  a.b2 = ADAM_B2;
+  a.eps = ADAM_EPS;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = TR;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(m->E * TR);
+  cfg.blockDim = dim3(TT);
+  cfg.dynamicSmemBytes = train_smem_bytes(m->in);
+  cfg.stream = m->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MCUDA(cudaLaunchKernelEx(&cfg, k_mlp_train, a));
+  return SPP_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -771,6 +1296,7 @@ int spp_mlp_create(int ensemble, int in_dim, SppMlp** out) {
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->mom, sizeof(float) * tot);
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->vel, sizeof(float) * tot);
   if (e == cudaSuccess) e = cudaMalloc((void**)&m->grad, sizeof(float) * tot);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&m->pub, sizeof(__nv_bfloat16) * (size_t)m->E * pub_size(in_dim));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
   {
     const char* env = getenv("SPP_MLP_SCALAR");
@@ -785,9 +1311,13 @@ int spp_mlp_create(int ensemble, int in_dim, SppMlp** out) {
   if (e == cudaSuccess) e = cudaMemset(m->mom, 0, sizeof(float) * tot);
   if (e == cudaSuccess) e = cudaMemset(m->vel, 0, sizeof(float) * tot);
   if (e != cudaSuccess) {
-    cudaFree(m->master); cudaFree(m->w); cudaFree(m->mom); cudaFree(m->vel); cudaFree(m->grad);
+    cudaFree(m->master); cudaFree(m->w); cudaFree(m->mom); cudaFree(m->vel); cudaFree(m->grad); cudaFree(m->pub);
     delete m;
     return mfail(SPP_ERR_ALLOC, std::string("mlp: ") + cudaGetErrorString(e));
+  }
+  {
+    const char* env = getenv("SPP_MLP_CLUSTER");   /* 0: the iteration graphs */
+    m->train_cluster = !(env && env[0] == '0') && train_cluster_fits(in_dim);
   }
   *out = m;
   return SPP_OK;
@@ -797,7 +1327,7 @@ int spp_mlp_destroy(SppMlp* m) {
   if (!m) return SPP_OK;
   cudaStreamSynchronize(m->stream);
   mlp_free_scratch(m);
-  cudaFree(m->master); cudaFree(m->w); cudaFree(m->mom); cudaFree(m->vel); cudaFree(m->grad);
+  cudaFree(m->master); cudaFree(m->w); cudaFree(m->mom); cudaFree(m->vel); cudaFree(m->grad); cudaFree(m->pub);
   cudaFree(m->bias); cudaFree(m->tix);
   cudaStreamDestroy(m->stream);
   delete m;
@@ -879,7 +1409,12 @@ int spp_mlp_train(SppMlp* m, const float* x, const float* t, const float* weight
     MCUDA(cudaMemcpyAsync(m->bias, table.data(), sizeof(float2) * iters, cudaMemcpyHostToDevice, m->stream));
     MCUDA(cudaMemsetAsync(m->tix, 0, sizeof(int), m->stream));
     int done = 0;
-    if (iters >= TRAIN_GRAPH_ITERS) {
+    if (train_in_cluster(m, B)) {
+      rc = mlp_train_cluster(m, B, iters, lr);
+      if (rc != SPP_OK) return rc;
+      done = iters;
+    }
+    if (iters - done >= TRAIN_GRAPH_ITERS) {
       cudaGraphExec_t exec;
       rc = mlp_train_graph(m, B, lr, &exec);
       if (rc != SPP_OK) return rc;

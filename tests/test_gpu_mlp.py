@@ -114,3 +114,26 @@ def test_tensor_core_and_scalar_kernels_agree(gpu_lib, monkeypatch):
     for e in range(3):
         assert np.linalg.norm(g0[e] - g1[e]) / np.linalg.norm(g1[e]) < 1e-5
     assert np.allclose(l0, l1, rtol=1e-5)
+
+
+@pytest.mark.parametrize("ensemble,in_dim,B", [(1, 1, 1), (2, 7, 15), (2, 16, 17), (9, 7, 303), (3, 7, 304),
+                                               (3, 16, 305), (1, 7, 513), (2, 3, 640)])
+def test_cluster_training_equals_the_iteration_graphs(gpu_lib, monkeypatch, ensemble, in_dim, B):
+    """Whole training calls in one cluster launch (k_mlp_train) keep the order
+    of every sum of the per-iteration kernels: the same parameters, bit for
+    bit, around the sizes of a tile (16 samples), a staged chunk (304), two
+    tiles per CTA (512) and more members than clusters fit at once."""
+    rng = np.random.default_rng(B)
+    x = rng.standard_normal((B, in_dim)).astype(np.float32)
+    t = np.tanh(x[:, 0]).astype(np.float32)
+    w = rng.uniform(0.5, 2, (ensemble, B)).astype(np.float32)
+    outs = []
+    for cluster in ("1", "0"):
+        monkeypatch.setenv("SPP_MLP_CLUSTER", cluster)
+        mlp = surrogate.Mlp(ensemble=ensemble, in_dim=in_dim, seed=5)
+        mlp.train(x, t, iters=1, lr=1e-2, weights=w)
+        loss = mlp.train(x, t, iters=53, lr=1e-3, weights=w)
+        outs.append((mlp.params(), loss, mlp.predict(x)))
+        mlp.close()
+    for a, b in zip(*outs):
+        assert np.array_equal(a, b)
