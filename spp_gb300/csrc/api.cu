@@ -91,7 +91,9 @@ struct SppSystem {
   int64_t step0 = 0;
   bool uploaded = false;
   bool use_graphs = true;
-  bool small_vicsek = false;     /* whole steps in one block (k_vicsek_small) */
+  VrunPlan vrun = {0, 0, 0, 0, 0, 0};   /* the same for the Vicsek models (k_vrun) */
+  VrunBufs vbuf = {};
+  char* vblock = nullptr;
   RunPlan run = {0, 0, 0};          /* resident runs (k_run): launch shape, 0 blocks = the step graphs */
   /* staging for uploads/downloads: x, y, theta, then the x and y counters
    * (int32), n entries each, in one device allocation */
@@ -99,6 +101,7 @@ struct SppSystem {
   float* stage_y = nullptr;
   float* stage_t = nullptr;
   int32_t* stage_img = nullptr;
+  char* block = nullptr;         /* every device array of d but the list, and stage_* */
   HostBlock* host = nullptr;     /* pinned: what a call reads back with one wait */
   std::vector<GraphEntry> graphs;
   /* tangent-space (Lyapunov) estimator */
@@ -131,6 +134,24 @@ int dalloc(T** ptr, size_t count) {
   return SPP_OK;
 }
 
+/* Several device arrays in one allocation (creating a system is mostly
+ * allocations: 30 of them cost 100 us more than one). */
+struct Arena {
+  std::vector<std::pair<void**, size_t>> parts;   /* where the address goes, offset */
+  size_t bytes = 0;
+  template <class T>
+  void want(T** ptr, size_t count) {
+    *ptr = nullptr;
+    parts.push_back({(void**)ptr, bytes});
+    bytes += ((count ? count : 1) * sizeof(T) + 255) / 256 * 256;
+  }
+  int take(char** block) {
+    int rc = dalloc(block, bytes);
+    for (auto& q : parts) *q.first = rc == SPP_OK ? (void*)(*block + q.second) : nullptr;
+    return rc;
+  }
+};
+
 void free_lyap(SppSystem* s) {
   LyapState& L = s->lyap;
   void* ptrs[] = {L.t0, L.ua, L.ub, L.acc, L.uslot, L.partial, L.rinv, L.log_stretch, L.error};
@@ -145,23 +166,49 @@ void free_lyap(SppSystem* s) {
   s->lyap_on = false;
 }
 
+void free_vrun(SppSystem* s) {
+  if (s->vblock) cudaFree(s->vblock);
+  s->vblock = nullptr;
+  s->vbuf = {};
+  s->vrun.blocks = 0;
+}
+
+/* The cell buckets of a resident Vicsek run.  Without the memory the system
+ * steps through the launches of the general path. */
+void alloc_vrun(SppSystem* s) {
+  VrunBufs& b = s->vbuf;
+  const size_t cells = s->vrun.cells, places = cells * s->vrun.cap;
+  b = {};
+  b.cells = s->vrun.cells;
+  b.cap = s->vrun.cap;
+  Arena arena;
+  for (int c = 0; c < 3; ++c) arena.want(&b.count[c], cells);
+  arena.want(&b.full, 3);
+  for (int c = 0; c < 2; ++c) {
+    arena.want(&b.bucket[c], places);
+    if (s->p.model == SPP_MODEL_VICSEK_REF_ANGLE) arena.want(&b.bucket_th[c], places);
+  }
+  if (arena.take(&s->vblock) != SPP_OK) {
+    cudaGetLastError();
+    free_vrun(s);
+  }
+}
+
 void free_dev(SppSystem* s) {
   if (s->mark_xy) cudaFree(s->mark_xy);
   if (s->mark_th) cudaFree(s->mark_th);
   s->mark_xy = nullptr;
   s->mark_th = nullptr;
   s->mark_step = -1;
-  DevState& d = s->d;
-  void* ptrs[] = {d.pos, d.half, d.half2, d.theta, d.img, d.id, d.inv, d.kacc, d.dth, d.ref, d.pos_alt,
-                  d.theta_alt, d.img_alt, d.id_alt, d.key, d.rank, d.cell_count, d.cell_start,
-                  d.scan_tmp, d.nbr, d.nn, d.long_q, d.nn_lanes, d.tumble, d.ctl, d.red, d.run_sums, s->stage_x};
-  for (void* q : ptrs)
-    if (q) cudaFree(q);
+  if (s->block) cudaFree(s->block);
+  if (s->d.nbr) cudaFree(s->d.nbr);
+  s->block = nullptr;
   memset(&s->d, 0, sizeof(s->d));
   s->stage_x = s->stage_y = s->stage_t = nullptr;
   s->stage_img = nullptr;
   if (s->host) cudaFreeHost(s->host);
   s->host = nullptr;
+  free_vrun(s);
 }
 
 double interaction_radius(const SppParams& p) { return spp_interaction_range(&p); }
@@ -275,10 +322,10 @@ int enqueue_rebuild(SppSystem* s, cudaStream_t st, int64_t* launches) {
 
 /* One step of the model, enqueued on st (stream or capture). */
 int enqueue_step(SppSystem* s, cudaStream_t st, bool capture, int64_t* launches) {
-  if (!s->uses_list && s->small_vicsek) {
-    if (launch_vicsek_small(s->k, s->d, 1, st, launches) != 0)
-      return fail(SPP_ERR_CUDA, "k_vicsek_small: cluster launch refused (shared memory or cluster shape)");
-    CUDA_TRY(cudaGetLastError());
+  if (s->vrun.blocks > 0) {
+    if (launch_vrun(s->k, s->d, s->vrun, s->vbuf, 1, 0, nullptr, st) != 0)
+      return fail(SPP_ERR_CUDA, std::string("k_vrun: ") + cudaGetErrorString(cudaGetLastError()));
+    if (launches) *launches += 1;
     return SPP_OK;
   }
   if (!s->uses_list) {
@@ -349,17 +396,36 @@ int get_graph(SppSystem* s, int nsteps, cudaGraphExec_t* out) {
   return SPP_OK;
 }
 
+/* Systems of up to 16,384 particles and fewer than 65,536 cells, with 24
+ * bytes per particle and 8 per cell within 224 KB. */
+bool vicsek_captures(const SppSystem* s) {
+  const size_t n = (size_t)s->d.n, cells = (size_t)s->d.D * s->d.D;
+  const size_t per_particle = s->p.model == SPP_MODEL_VICSEK_REF_ANGLE ? 24 : 20;
+  return n <= 16384 && cells < 65536 && per_particle * n + 8 * cells <= 224 * 1024;
+}
+
+/* nsteps steps of a resident Vicsek run, in launches of whole frames. */
+int run_vicsek(SppSystem* s, int64_t nsteps, int every, unsigned long long* sums) {
+  const int64_t unit = every > 0 ? every : 1;
+  const int64_t most = RUN_CHUNK / unit > 0 ? RUN_CHUNK / unit * unit : unit;
+  while (nsteps > 0) {
+    const int chunk = (int)(nsteps > most ? most : nsteps);
+    if (launch_vrun(s->k, s->d, s->vrun, s->vbuf, chunk, every, sums, s->stream) != 0)
+      return fail(SPP_ERR_CUDA, std::string("k_vrun: ") + cudaGetErrorString(cudaGetLastError()));
+    s->host_launches++;
+    if (sums) sums += 2 * (chunk / unit);
+    nsteps -= chunk;
+  }
+  return SPP_OK;
+}
+
 int run_steps(SppSystem* s, int64_t nsteps) {
-  if (s->small_vicsek) {
-    /* one launch per call runs every step */
-    while (nsteps > 0) {
-      const int chunk = nsteps > (1 << 20) ? (1 << 20) : (int)nsteps;
-      if (launch_vicsek_small(s->k, s->d, chunk, s->stream, &s->host_launches) != 0)
-        return fail(SPP_ERR_CUDA, "k_vicsek_small: cluster launch refused (shared memory or cluster shape)");
-      CUDA_TRY(cudaGetLastError());
-      nsteps -= chunk;
-    }
-    return SPP_OK;
+  if (s->vrun.blocks > 0) {
+    /* a stream that is being captured takes small systems (one launch per
+     * call); the others go to the step graphs, whose own capture it refuses */
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CUDA_TRY(cudaStreamIsCapturing(s->stream, &cs));
+    if (cs == cudaStreamCaptureStatusNone || vicsek_captures(s)) return run_vicsek(s, nsteps, 0, nullptr);
   }
   if (!s->use_graphs) {
     for (int64_t i = 0; i < nsteps; ++i) {
@@ -636,6 +702,14 @@ int spp_internal_view(SppSystem* s, DevState* d, SppConsts* k, cudaStream_t* st)
   return SPP_OK;
 }
 
+int spp_internal_series(SppSystem* s, int nframes, int every, unsigned long long* sums) {
+  if (s->vrun.blocks <= 0) return 1;
+  const int64_t nsteps = (int64_t)nframes * every;
+  if (s->target_step + nsteps > 0xffffffffLL) return fail(SPP_ERR_INVALID, "step counter overflow"), -1;
+  s->target_step += nsteps;
+  return run_vicsek(s, nsteps, every, sums) == SPP_OK ? 0 : -2;
+}
+
 void spp_internal_count_launches(SppSystem* s, int n) {
   if (s) s->host_launches += n;
 }
@@ -783,10 +857,6 @@ int spp_create(const SppParams* p, SppSystem** out) {
   d.D = D;
   d.morton_bits = bits;
   d.n_keys = 1u << (2 * bits);
-  {
-    const char* sv = getenv("SPP_VICSEK_SMALL");
-    s->small_vicsek = !s->uses_list && !(sv && sv[0] == '0') && vicsek_small_fits(s->k, d);
-  }
   int cap = p->list_capacity > 0 ? p->list_capacity : list_capacity_for(*p, rcell);
   if (!s->uses_list) cap = 0;
   size_t n = (size_t)p->n;
@@ -795,34 +865,35 @@ int spp_create(const SppParams* p, SppSystem** out) {
     delete s;
     return fail(SPP_ERR_INVALID, "cell grid too large for the scan");
   }
-  rc = SPP_OK;
-  rc = rc ? rc : dalloc(&d.pos, n);
-  rc = rc ? rc : dalloc(&d.half, s->uses_list ? n : 1);
-  rc = rc ? rc : dalloc(&d.half2, s->nstages > 2 ? n : 1);
-  rc = rc ? rc : dalloc(&d.theta, n);
-  rc = rc ? rc : dalloc(&d.img, n);
-  rc = rc ? rc : dalloc(&d.id, n);
-  if (p->model == SPP_MODEL_BEADS) rc = rc ? rc : dalloc(&d.inv, n);
-  if (s->k.tumble) rc = rc ? rc : dalloc(&d.tumble, n);
-  rc = rc ? rc : dalloc(&d.kacc, s->nstages > 2 ? n : 1);
-  rc = rc ? rc : dalloc(&d.dth, s->nstages > 1 ? n : 1);
-  rc = rc ? rc : dalloc(&d.ref, n);
-  rc = rc ? rc : dalloc(&d.pos_alt, n);
-  rc = rc ? rc : dalloc(&d.theta_alt, n);
-  rc = rc ? rc : dalloc(&d.img_alt, n);
-  rc = rc ? rc : dalloc(&d.id_alt, n);
-  rc = rc ? rc : dalloc(&d.key, n);
-  rc = rc ? rc : dalloc(&d.rank, n);
-  rc = rc ? rc : dalloc(&d.cell_count, d.n_keys);
-  rc = rc ? rc : dalloc(&d.cell_start, d.n_keys);
-  rc = rc ? rc : dalloc(&d.scan_tmp, nscan);
-  rc = rc ? rc : dalloc(&d.nn, n);
-  rc = rc ? rc : dalloc(&d.long_q, n);
-  if (s->k.lanes > 1) rc = rc ? rc : dalloc(&d.nn_lanes, n);
-  rc = rc ? rc : dalloc(&d.ctl, 1);
-  rc = rc ? rc : dalloc(&d.red, 4);
-  rc = rc ? rc : dalloc(&d.run_sums, s->uses_list ? RUN_MAX_BLOCKS : 1);
-  rc = rc ? rc : dalloc(&s->stage_x, 5 * n);
+  Arena arena;
+  arena.want(&d.pos, n);
+  arena.want(&d.half, s->uses_list ? n : 1);
+  arena.want(&d.half2, s->nstages > 2 ? n : 1);
+  arena.want(&d.theta, n);
+  arena.want(&d.img, n);
+  arena.want(&d.id, n);
+  if (p->model == SPP_MODEL_BEADS) arena.want(&d.inv, n);
+  if (s->k.tumble) arena.want(&d.tumble, n);
+  arena.want(&d.kacc, s->nstages > 2 ? n : 1);
+  arena.want(&d.dth, s->nstages > 1 ? n : 1);
+  arena.want(&d.ref, n);
+  arena.want(&d.pos_alt, n);
+  arena.want(&d.theta_alt, n);
+  arena.want(&d.img_alt, n);
+  arena.want(&d.id_alt, n);
+  arena.want(&d.key, n);
+  arena.want(&d.rank, n);
+  arena.want(&d.cell_count, d.n_keys);
+  arena.want(&d.cell_start, d.n_keys);
+  arena.want(&d.scan_tmp, nscan);
+  arena.want(&d.nn, n);
+  arena.want(&d.long_q, n);
+  if (s->k.lanes > 1) arena.want(&d.nn_lanes, n);
+  arena.want(&d.ctl, 1);
+  arena.want(&d.red, 4);
+  arena.want(&d.run_sums, RUN_MAX_BLOCKS);
+  arena.want(&s->stage_x, 5 * n);
+  rc = arena.take(&s->block);
   if (rc == SPP_OK) {
     s->stage_y = s->stage_x + n;
     s->stage_t = s->stage_x + 2 * n;
@@ -850,7 +921,10 @@ int spp_create(const SppParams* p, SppSystem** out) {
   s->own_stream = true;
   {
     const char* rv = getenv("SPP_RESIDENT");
-    if (s->uses_list && !(rv && rv[0] == '0')) plan_run(s->k, d, &s->run);
+    const char* sv = getenv("SPP_VICSEK_SMALL");
+    const bool off = rv && rv[0] == '0';
+    if (s->uses_list && !off) plan_run(s->k, d, &s->run);
+    if (!s->uses_list && !off && !(sv && sv[0] == '0') && plan_vrun(s->k, d, &s->vrun)) alloc_vrun(s);
   }
   s->per_rebuild_kernels = 7;   /* bin_count, scan x3, scatter, build_list, sort_long */
   s->per_step_kernels = s->uses_list ? (s->nstages == 1 ? 2 : s->nstages) : 6;

@@ -29,6 +29,7 @@
  * persistent grid was slower, 35.7 against 33.8 us per stage).
  */
 #include "spp_internal.cuh"
+#include "spp_grid.cuh"
 #include "spp_list.cuh"
 
 namespace {
@@ -64,41 +65,11 @@ struct Cold<2> {
   __device__ __forceinline__ Cold(float* c, int s) : col(c), stride(s) {}
   __device__ __forceinline__ float& operator[](int q) { return col[q * stride]; }
 };
-/* polls of a barrier's counter before a block gives up (a poll takes about
- * 0.7 us: seconds; a barrier is normally met within microseconds) */
-constexpr int RUN_WAIT_LIMIT = 1 << 22;
 /* Neighbour states gathered together.  Measured (us per RK2 / RK4 step, ABP
  * at unit density, groups of 2 / 4): one lane, one block per SM, N = 65,536:
  * 10.35 / 10.01 and 18.2 / 17.4; two blocks per SM (56 registers), N =
  * 163,840: 14.5 / 15.2 and 24.4 / 25.8; four lanes, N = 16,384: 8.6 / 8.7. */
 __host__ __device__ constexpr int run_group(int lanes, int per_sm) { return lanes == 1 && per_sm == 1 ? 4 : 2; }
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-/* One arrival of the block at the grid barrier: every write of the block
- * before it is visible to a block that has waited for it.  Thread 0 calls,
- * after a __syncthreads. */
-__device__ __forceinline__ void grid_arrive(Ctl* ctl) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->run_bar) : "memory");
-}
-
-/* Thread 0: waits until the counter has reached target, or gives up. */
-__device__ __forceinline__ bool grid_wait(Ctl* ctl, unsigned target) {
-  for (int it = 0; it < RUN_WAIT_LIMIT; ++it)
-    if (ld_acquire(&ctl->run_bar) >= target) return true;
-  atomicOr(&ctl->run_timeout, 1u);
-  return false;
-}
 
 template <int LAW, int KIND>
 __device__ __forceinline__ void run_pair(const SppConsts& k, const DevState& d, int wrap, SppAccF* a, int nbi, int j,
@@ -192,39 +163,7 @@ __device__ __noinline__ int run_rebuild(const SppConsts& k, const DevState& d, i
     }
   }
   if (!barrier()) return RUN_LOST;
-  /* exclusive scan of the cell counts: each block sums, then scans, its own
-   * range of cells (a multiple of 4 for 16-byte loads; n_keys is a power of
-   * 4, at least 16) */
-  const uint32_t per_block = ((d.n_keys + gridDim.x - 1) / gridDim.x + 3u) & ~3u;
-  const uint32_t c0 = min(per_block * blockIdx.x, d.n_keys), c1 = min(c0 + per_block, d.n_keys);
-  {
-    uint32_t sum = 0u;
-    for (uint32_t c = c0 + 4u * tid; c < c1; c += 4u * T) {
-      const uint4 v = *reinterpret_cast<const uint4*>(d.cell_count + c);
-      sum += (v.x + v.y) + (v.z + v.w);
-    }
-    uint32_t total;
-    block_exclusive_scan(sum, &total);
-    if (tid == 0) d.run_sums[blockIdx.x] = total;
-  }
-  if (!barrier()) return RUN_LOST;
-  {
-    uint32_t before = 0u;
-    for (uint32_t b = tid; b < blockIdx.x; b += T) before += d.run_sums[b];
-    uint32_t carry;
-    block_exclusive_scan(before, &carry);
-    for (uint32_t cb = c0; cb < c1; cb += 4u * T) {
-      __syncthreads();
-      const uint32_t c = cb + 4u * tid;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (c < c1) v = *reinterpret_cast<const uint4*>(d.cell_count + c);
-      uint32_t total;
-      const uint32_t e = carry + block_exclusive_scan((v.x + v.y) + (v.z + v.w), &total);
-      if (c < c1)
-        *reinterpret_cast<uint4*>(d.cell_start + c) = make_uint4(e, e + v.x, e + v.x + v.y, e + v.x + v.y + v.z);
-      carry += total;
-    }
-  }
+  if (!grid_scan(d.cell_count, d.cell_start, d.n_keys, d.run_sums, barrier)) return RUN_LOST;
   if (!barrier()) return RUN_LOST;
   if (head) {
     const uint32_t dst = d.cell_start[key] + rank;

@@ -362,7 +362,12 @@ int spp_polarization_series(SppSystem* s, int nframes, int every, double* p, dou
    * wait for the steps (re-run by spp_sync) before P is read.  The Vicsek
    * models have no list: their frames queue up without host round trips. */
   const bool listed = k.model == SPP_MODEL_ABP || k.model == SPP_MODEL_CONTINUOUS || k.model == SPP_MODEL_BEADS;
-  for (int f = 0; f < nframes && rc == SPP_OK && e == cudaSuccess; ++f) {
+  int whole = 1;   /* 0: every frame in one resident run */
+  if (e == cudaSuccess) {
+    whole = spp_internal_series(s, nframes, every, sums);
+    if (whole < 0) rc = whole == -1 ? SPP_ERR_INVALID : SPP_ERR_CUDA;
+  }
+  for (int f = 0; whole > 0 && f < nframes && rc == SPP_OK && e == cudaSuccess; ++f) {
     rc = spp_step(s, every);
     if (rc == SPP_OK && listed) rc = spp_sync(s);
     if (rc == SPP_OK) {

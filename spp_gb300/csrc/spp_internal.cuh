@@ -109,6 +109,9 @@ void spp_internal_count_launches(SppSystem* s, int n);
 /* api.cu: the marked-frame buffers of spp_ring_motion (n entries each, by
  * particle id; allocated on first use) and the mark's step (-1: none) */
 int spp_internal_mark(SppSystem* s, double2** xy, float** th, int64_t** step);
+/* api.cu: nframes x every steps of a resident Vicsek run with the heading
+ * sums of every frame; 1: not such a system, < 0: error (message set) */
+int spp_internal_series(SppSystem* s, int nframes, int every, unsigned long long* sums);
 /* api.cu: the absolute step counter (waits for the stream); -1 on error */
 int64_t spp_internal_step(SppSystem* s);
 /* api.cu: the time step as given (double) */
@@ -155,15 +158,27 @@ struct RunPlan {
 };
 bool plan_run(const SppConsts& k, const DevState& d, RunPlan* plan);
 int launch_run(const SppConsts& k, const DevState& d, const RunPlan& plan, int nstages, int nsteps, cudaStream_t s);
+/* kernels_vrun.cu: the same for the discrete Vicsek models.  every > 0: the
+ * fixed-point heading sums after every `every` steps are added into sums
+ * (two words per frame, zeroed by the caller). */
+struct VrunPlan {
+  int blocks, threads;    /* 0 blocks: the system does not fit */
+  int lanes, per_sm;
+  uint32_t cells;         /* D * D, rounded up to a multiple of 4 */
+  int cap;                /* places per cell bucket */
+};
+struct VrunBufs {
+  uint32_t* count[3];
+  uint32_t* full;         /* [3] */
+  float4* bucket[2];      /* [cells][cap] */
+  float* bucket_th[2];    /* headings, angle rule only */
+  uint32_t cells;
+  int cap;
+};
+bool plan_vrun(const SppConsts& k, const DevState& d, VrunPlan* plan);
+int launch_vrun(const SppConsts& k, const DevState& d, const VrunPlan& plan, const VrunBufs& vb, int nsteps, int every,
+                unsigned long long* sums, cudaStream_t s);
 void launch_vicsek_step(const SppConsts& k, const DevState& d, cudaStream_t s, int64_t* launches);
-/* Whole Vicsek steps of a small system in one thread-block cluster
- * (k_vicsek_small): at most SPP_SMALL_MAX_N particles, fewer than 65536
- * cells, and SPP_SMALL_MAX_SMEM bytes of cell-ordered copy plus cell table
- * per CTA. */
-#define SPP_SMALL_MAX_N 16384
-#define SPP_SMALL_MAX_SMEM (224 * 1024)
-bool vicsek_small_fits(const SppConsts& k, const DevState& d);
-int launch_vicsek_small(const SppConsts& k, const DevState& d, int nsteps, cudaStream_t s, int64_t* launches);
 void launch_polarization(const DevState& d, cudaStream_t s);
 /* the two fixed-point heading sums added into sums[0..1] (zeroed by the caller) */
 void launch_polarization_into(const DevState& d, unsigned long long* sums, cudaStream_t s);

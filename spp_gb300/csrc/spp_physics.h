@@ -723,6 +723,16 @@ SPP_HD void spp_euler_update(float x0, float y0, float th0, float fx, float fy, 
 /* ------------------------------------------------------------------ */
 /* Vicsek family                                                       */
 /* ------------------------------------------------------------------ */
+/* VicsekParticle2's push between close particles (shared/particle.h:233-244). */
+SPP_HD void spp_push_vicsek(const SppConsts* k, SppAcc* a, float dx, float dy, float d2) {
+  const float r = spp_rsqrtf(d2);
+  const float d = d2 * r;
+  float fa = k->beta_push / (1.0f + spp_expf(d / k->r_push - 2.0f));
+  float t = fa * r;
+  spp_fx_add_guarded(&a->ax, t * dx, &a->ovf);
+  spp_fx_add_guarded(&a->ay, t * dy, &a->ovf);
+}
+
 /* Configured rule: sum e^{i theta_j} over |r_ij| < r, self included (the
  * self term comes from the d2 = 0 visit of j = i). */
 SPP_HD void spp_pair_vicsek(const SppConsts* k, SppAcc* a, float xi, float yi, float xj, float yj,
@@ -750,14 +760,7 @@ SPP_HD void spp_pair_vicsek(const SppConsts* k, SppAcc* a, float xi, float yi, f
     a->cnt += 1;
     spp_fx_add(&a->ax, cj);
     spp_fx_add(&a->ay, sj);
-    if (d2 < k->rpush2 && d2 > 0.0f) {
-      const float r = spp_rsqrtf(d2);
-      const float d = d2 * r;
-      float fa = k->beta_push / (1.0f + spp_expf(d / k->r_push - 2.0f));
-      float t = fa * r;
-      spp_fx_add_guarded(&a->ax, t * dx, &a->ovf);
-      spp_fx_add_guarded(&a->ay, t * dy, &a->ovf);
-    }
+    if (d2 < k->rpush2 && d2 > 0.0f) spp_push_vicsek(k, a, dx, dy, d2);
   }
 }
 
