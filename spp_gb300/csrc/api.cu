@@ -87,6 +87,11 @@ struct SppSystem {
   double2* mark_xy = nullptr;
   float* mark_th = nullptr;
   int64_t mark_step = -1;
+  /* scratch of the pair statistics (spp_internal_obs_space), grown on use */
+  uint32_t* obs_grid = nullptr;
+  size_t obs_cells = 0;
+  unsigned long long* obs_bins = nullptr;
+  size_t obs_nbins = 0;
   int64_t target_step = 0;       /* step the caller has asked to reach */
   int64_t step0 = 0;
   bool uploaded = false;
@@ -200,6 +205,11 @@ void free_dev(SppSystem* s) {
   s->mark_xy = nullptr;
   s->mark_th = nullptr;
   s->mark_step = -1;
+  if (s->obs_grid) cudaFree(s->obs_grid);
+  if (s->obs_bins) cudaFree(s->obs_bins);
+  s->obs_grid = nullptr;
+  s->obs_bins = nullptr;
+  s->obs_cells = s->obs_nbins = 0;
   if (s->block) cudaFree(s->block);
   if (s->d.nbr) cudaFree(s->d.nbr);
   s->block = nullptr;
@@ -723,6 +733,33 @@ int spp_internal_mark(SppSystem* s, double2** xy, float** th, int64_t** step) {
   *xy = s->mark_xy;
   *th = s->mark_th;
   *step = &s->mark_step;
+  return SPP_OK;
+}
+
+int spp_internal_obs_space(SppSystem* s, size_t cells, size_t bins, uint32_t** count, uint32_t** start, uint32_t** tmp,
+                           unsigned long long** counts) {
+  if (cells > s->d.n_keys && cells > s->obs_cells) {
+    if (s->obs_grid) cudaFree(s->obs_grid);
+    s->obs_grid = nullptr;
+    s->obs_cells = 0;
+    const size_t padded = (cells + 63) / 64 * 64;
+    int rc = dalloc(&s->obs_grid, 2 * padded + cells / 4096 + 2);
+    if (rc != SPP_OK) return rc;
+    s->obs_cells = padded;
+  }
+  if (bins > s->obs_nbins) {
+    if (s->obs_bins) cudaFree(s->obs_bins);
+    s->obs_bins = nullptr;
+    s->obs_nbins = 0;
+    int rc = dalloc(&s->obs_bins, bins);
+    if (rc != SPP_OK) return rc;
+    s->obs_nbins = bins;
+  }
+  const bool own = cells > s->d.n_keys;
+  *count = own ? s->obs_grid : s->d.cell_count;
+  *start = own ? s->obs_grid + s->obs_cells : s->d.cell_start;
+  *tmp = own ? s->obs_grid + 2 * s->obs_cells : s->d.scan_tmp;
+  *counts = s->obs_bins;
   return SPP_OK;
 }
 

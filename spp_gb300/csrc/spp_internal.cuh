@@ -109,6 +109,11 @@ void spp_internal_count_launches(SppSystem* s, int n);
 /* api.cu: the marked-frame buffers of spp_ring_motion (n entries each, by
  * particle id; allocated on first use) and the mark's step (-1: none) */
 int spp_internal_mark(SppSystem* s, double2** xy, float** th, int64_t** step);
+/* api.cu: scratch of the pair statistics, kept with the system: counts and
+ * starts of `cells` cells with the scan's block sums (the rebuild's own
+ * arrays where they are large enough), and `bins` 64-bit counts */
+int spp_internal_obs_space(SppSystem* s, size_t cells, size_t bins, uint32_t** count, uint32_t** start, uint32_t** tmp,
+                           unsigned long long** counts);
 /* api.cu: nframes x every steps of a resident Vicsek run with the heading
  * sums of every frame; 1: not such a system, < 0: error (message set) */
 int spp_internal_series(SppSystem* s, int nframes, int every, unsigned long long* sums);
