@@ -111,6 +111,8 @@ struct SppSystem {
   std::vector<GraphEntry> graphs;
   /* tangent-space (Lyapunov) estimator */
   LyapState lyap;
+  RunPlan lrun = {0, 0, 0};      /* resident Lyapunov runs (k_lrun) */
+  char* lyap_block = nullptr;    /* the arrays of `lyap` */
   bool lyap_on = false;
   int64_t lyap_steps = 0;        /* steps since spp_lyap_init */
   int lyap_renorm_every = 10;
@@ -159,9 +161,9 @@ struct Arena {
 
 void free_lyap(SppSystem* s) {
   LyapState& L = s->lyap;
-  void* ptrs[] = {L.t0, L.ua, L.ub, L.acc, L.uslot, L.partial, L.rinv, L.log_stretch, L.error};
-  for (void* q : ptrs)
-    if (q) cudaFree(q);
+  if (s->lyap_block) cudaFree(s->lyap_block);
+  s->lyap_block = nullptr;
+  s->lrun.blocks = 0;
   memset(&L, 0, sizeof(L));
   for (auto& g : s->lyap_graphs) {
     cudaGraphExecDestroy(g.exec);
@@ -688,6 +690,19 @@ int get_lyap_graph(SppSystem* s, int chunk, cudaGraphExec_t* out) {
 int launch_lyap_chunks(SppSystem* s, int64_t nsteps) {
   const int every = s->lyap_renorm_every > 0 ? s->lyap_renorm_every : 10;
   int64_t left = nsteps;
+  if (s->lrun.blocks > 0) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CUDA_TRY(cudaStreamIsCapturing(s->stream, &cs));
+    const int64_t most = RUN_CHUNK / every > 0 ? (int64_t)(RUN_CHUNK / every) * every : every;
+    while (cs == cudaStreamCaptureStatusNone && left > 0) {
+      const int part = (int)(left > most ? most : left);
+      if (launch_lrun(s->k, s->d, s->lyap, s->lrun, s->nstages, part, every, s->stream) != 0)
+        return fail(SPP_ERR_CUDA, std::string("k_lrun: ") + cudaGetErrorString(cudaGetLastError()));
+      /* the passes that the step graphs would launch */
+      s->graph_kernels += (int64_t)part * (2 * s->nstages + 1) + 6 * ((part + every - 1) / every);
+      left -= part;
+    }
+  }
   while (left > 0) {
     int chunk = left >= every ? every : (int)left;
     cudaGraphExec_t exec;
@@ -1309,21 +1324,28 @@ int spp_lyap_init(SppSystem* s, int K, uint64_t seed) {
   if (s->nstages < 2) return fail(SPP_ERR_UNSUPPORTED, "tangent dynamics needs RK2 or RK4");
   int rc = spp_sync(s);
   if (rc != SPP_OK) return rc;
-  free_lyap(s);
   LyapState& L = s->lyap;
-  L.K = K;
-  L.n = s->p.n;
-  size_t len = (size_t)K * 3 * s->p.n;
-  rc = dalloc(&L.t0, len);
-  rc = rc ? rc : dalloc(&L.ua, len);
-  rc = rc ? rc : dalloc(&L.ub, len);
-  rc = rc ? rc : dalloc(&L.acc, len);
-  rc = rc ? rc : dalloc(&L.uslot, 2 * tangent_slot_floats(K, s->p.n));
-  rc = rc ? rc : dalloc(&L.partial, (size_t)SPP_GRAM_BLOCKS * SPP_GRAM_ENTRIES);
-  rc = rc ? rc : dalloc(&L.rinv, (size_t)SPP_LYAP_MAX * SPP_LYAP_MAX);
-  rc = rc ? rc : dalloc(&L.log_stretch, SPP_LYAP_MAX);
-  rc = rc ? rc : dalloc(&L.error, 1);
-  if (rc != SPP_OK) { free_lyap(s); return rc; }
+  s->lyap_on = false;
+  if (!s->lyap_block || L.K != K) {
+    free_lyap(s);
+    const size_t len = (size_t)K * 3 * s->p.n;
+    Arena arena;
+    arena.want(&L.t0, len);
+    arena.want(&L.ua, len);
+    arena.want(&L.ub, len);
+    arena.want(&L.acc, len);
+    arena.want(&L.uslot, 2 * tangent_slot_floats(K, s->p.n));
+    arena.want(&L.partial, (size_t)SPP_GRAM_BLOCKS * SPP_GRAM_ENTRIES);
+    arena.want(&L.rinv, (size_t)SPP_LYAP_MAX * SPP_LYAP_MAX);
+    arena.want(&L.log_stretch, SPP_LYAP_MAX);
+    arena.want(&L.error, 1);
+    rc = arena.take(&s->lyap_block);
+    if (rc != SPP_OK) { free_lyap(s); return rc; }
+    L.K = K;
+    L.n = s->p.n;
+    const char* rv = getenv("SPP_RESIDENT");
+    if (!(rv && rv[0] == '0')) plan_lrun(s->k, s->d, K, &s->lrun);
+  }
   CUDA_TRY(cudaMemsetAsync(L.log_stretch, 0, sizeof(double) * SPP_LYAP_MAX, s->stream));
   CUDA_TRY(cudaMemsetAsync(L.error, 0, sizeof(uint32_t), s->stream));
   CUDA_TRY(cudaMemsetAsync(L.uslot, 0, 2 * sizeof(float) * tangent_slot_floats(K, s->p.n), s->stream));
