@@ -19,6 +19,15 @@
  * instead of 64, and the factorisation runs in a warp (right-looking, one
  * entry per lane, each entry's subtractions in the order of
  * spp_cholesky_inverse) in every block redundantly, which saves a barrier.
+ *
+ * Measured (one GB300, N = 16,384, K = 8, RK4, renormalised every 10 steps; us
+ * per step, step graphs -> this): uniform 85 -> 31, flocked (60% of the
+ * particles in flocks, lists of up to 159) 113 -> 61.  The renormalisation is
+ * about 5 us of a step; the rest is the chain of k_run's stages (barrier,
+ * gathers of 48 bytes per neighbour, update) and, in flocks, the longest
+ * segments.  Flocked, 3 / 4 / 6 neighbours in flight in long segments 68 / 71 /
+ * 73 (2: 76), dealing the warps around the blocks 68 -> 61; at unit density
+ * dealing costs 3%, so short lists keep consecutive slots.
  */
 #include "spp_rebuild.cuh"
 #include "spp_lyap.cuh"
@@ -188,18 +197,24 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
     k_lrun(const __grid_constant__ SppConsts k, const __grid_constant__ DevState d, const __grid_constant__ LyapState L,
            int nst, int nsteps, int every) {
   constexpr int VPL = KP / LANES;          /* vectors per lane: v = lane_r + LANES m */
-  constexpr int GROUP = LANES == 1 ? 3 : 2;
+  constexpr int GROUP = LANES == 1 ? 3 : 2;   /* neighbours gathered together */
+  constexpr int BIG = 3;                      /* the same for long segments */
   extern __shared__ __align__(16) unsigned char lrun_smem[];
   __shared__ unsigned fin[2][2];
   __shared__ unsigned s_word;
   __shared__ CholShared chol;
   __shared__ double warp_part[SPP_GRAM_THREADS / 32][SPP_GRAM_ENTRIES];
   const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
-  int32_t* const rows = reinterpret_cast<int32_t*>(lrun_smem) + tid;                        /* [RUN_ROWS][T] */
+  const int R = run_rows(d.cap, LANES, 1);
+  int32_t* const rows = reinterpret_cast<int32_t*>(lrun_smem) + tid;                        /* [R][T] */
   unsigned long long* const keycol = reinterpret_cast<unsigned long long*>(lrun_smem) + tid; /* [LIST_LOCAL][T] */
   Ctl* const ctl = d.ctl;
   const int n = d.n, K = L.K;
-  const int i = (blockIdx.x * T + tid) / LANES;
+  /* Consecutive slots to consecutive threads; with long lists warp by warp
+   * around the blocks, so that a flock's particles (neighbours in the slot
+   * order) are spread over the SMs. */
+  const int i = (R > RUN_ROWS ? ((tid >> 5) * (int)gridDim.x + (int)blockIdx.x) * 32 + lane : (int)blockIdx.x * T + tid) /
+                LANES;
   const int lane_r = LANES == 1 ? 0 : tid % LANES;
   const bool inb = i < n;
   const bool head = inb && lane_r == 0;
@@ -232,7 +247,8 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
   }
   const float* us = L.uslot;                                 /* [n][KP], this stage's */
   float* uo = L.uslot + (size_t)KP * (size_t)n;              /* the next stage's */
-  auto load = [&](bool with_list) {
+  bool wide = false;
+  auto load_own = [&](bool with_list) {
     if (!inb) return;
     p = d.pos[i];
     pid = d.id[i];
@@ -246,7 +262,7 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
       for (int r = 0; r < lane_r; ++r) q_begin += (int)((lc >> (16 * r)) & 0xffffull);
       len = (int)((lc >> (16 * lane_r)) & 0xffffull);
     }
-    const int mr = len < RUN_ROWS ? len : RUN_ROWS;
+    const int mr = len < R ? len : R;
     for (int q = 0; q < mr; q += 4) {
       int v[4];
 #pragma unroll
@@ -255,6 +271,10 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
       for (int w = 0; w < 4; ++w)
         if (q + w < mr) rows[(q + w) * T] = spp_index_ok(ctl, v[w], n) ? v[w] : i;
     }
+  };
+  auto load = [&](bool with_list) {
+    load_own(with_list);
+    wide = __reduce_max_sync(0xffffffffu, (unsigned)len) >= (unsigned)RUN_LONG;
   };
   /* the owner's vectors from and to L.t0 (by particle id) */
   auto fetch_vectors = [&]() {
@@ -329,15 +349,50 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
 #pragma unroll
       for (int g = 0; g < KP / 4; ++g)
         ui[g] = inb ? reinterpret_cast<const float4*>(us + (size_t)i * KP)[g] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      for (int q0 = 0; q0 < len; q0 += GROUP) {
+      /* one neighbour: the base stage's alignment sums and the vectors'
+       * couplings */
+      auto pair = [&](const float4& pj, const float4* uj) {
+        float dx, dy;
+        const float d2 = plain ? spp_pair_sep(&k, 0, p.x, p.y, pj.x, pj.y, &dx, &dy)
+                               : spp_pair_sep(&k, 1, p.x, p.y, pj.x, pj.y, &dx, &dy);
+        if (!(d2 < k.ral2)) return;
+        const spp_f2 cs = spp_add2(spp_f2_make(a.sc, a.ss), spp_f2_make(pj.z, pj.w));
+        a.sc = cs.x;
+        a.ss = cs.y;
+        const float cij = spp_tangent_coupling(p.z, p.w, pj.z, pj.w);
+#pragma unroll
+        for (int g = 0; g < KP / 4; ++g) {
+          acc[4 * g] = acc[4 * g] + cij * (uj[g].x - ui[g].x);
+          acc[4 * g + 1] = acc[4 * g + 1] + cij * (uj[g].y - ui[g].y);
+          acc[4 * g + 2] = acc[4 * g + 2] + cij * (uj[g].z - ui[g].z);
+          acc[4 * g + 3] = acc[4 * g + 3] + cij * (uj[g].w - ui[g].w);
+        }
+      };
+      auto entry = [&](int q) -> int {
+        const int j = q < R ? rows[q * T] : d.nbr[(size_t)(q_begin + q) * n + i];
+        return spp_index_ok(ctl, j, n) ? j : i;
+      };
+      int q0 = 0;
+      if (wide)
+        for (; q0 + BIG <= len; q0 += BIG) {
+          int jg[BIG];
+          float4 pg[BIG], ug[BIG][KP / 4];
+#pragma unroll
+          for (int w = 0; w < BIG; ++w) jg[w] = entry(q0 + w);
+#pragma unroll
+          for (int w = 0; w < BIG; ++w) {
+            pg[w] = cur[jg[w]];
+#pragma unroll
+            for (int g = 0; g < KP / 4; ++g) ug[w][g] = reinterpret_cast<const float4*>(us + (size_t)jg[w] * KP)[g];
+          }
+#pragma unroll
+          for (int w = 0; w < BIG; ++w) pair(pg[w], ug[w]);
+        }
+      for (; q0 < len; q0 += GROUP) {
         int jg[GROUP];
         float4 pg[GROUP], ug[GROUP][KP / 4];
 #pragma unroll
-        for (int w = 0; w < GROUP; ++w) {
-          const int q = q0 + w;
-          jg[w] = q < len ? (q < RUN_ROWS ? rows[q * T] : d.nbr[(size_t)(q_begin + q) * n + i]) : i;
-          if (!spp_index_ok(ctl, jg[w], n)) jg[w] = i;
-        }
+        for (int w = 0; w < GROUP; ++w) jg[w] = q0 + w < len ? entry(q0 + w) : i;
 #pragma unroll
         for (int w = 0; w < GROUP; ++w) {
           pg[w] = cur[jg[w]];
@@ -346,25 +401,7 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
         }
 #pragma unroll
         for (int w = 0; w < GROUP; ++w)
-          if (q0 + w < len) {
-            float dx, dy;
-            const float d2 = plain ? spp_pair_sep(&k, 0, p.x, p.y, pg[w].x, pg[w].y, &dx, &dy)
-                                   : spp_pair_sep(&k, 1, p.x, p.y, pg[w].x, pg[w].y, &dx, &dy);
-            if (d2 < k.ral2) {
-              /* the base stage's alignment sums and the vectors' couplings */
-              const spp_f2 cs = spp_add2(spp_f2_make(a.sc, a.ss), spp_f2_make(pg[w].z, pg[w].w));
-              a.sc = cs.x;
-              a.ss = cs.y;
-              const float cij = spp_tangent_coupling(p.z, p.w, pg[w].z, pg[w].w);
-#pragma unroll
-              for (int g = 0; g < KP / 4; ++g) {
-                acc[4 * g] = acc[4 * g] + cij * (ug[w][g].x - ui[g].x);
-                acc[4 * g + 1] = acc[4 * g + 1] + cij * (ug[w][g].y - ui[g].y);
-                acc[4 * g + 2] = acc[4 * g + 2] + cij * (ug[w][g].z - ui[g].z);
-                acc[4 * g + 3] = acc[4 * g + 3] + cij * (ug[w][g].w - ui[g].w);
-              }
-            }
-          }
+          if (q0 + w < len) pair(pg[w], ug[w]);
       }
       /* lane sums as (p0 + p1) + (p2 + p3); each lane keeps its own vectors' */
       float mine[VPL];
@@ -570,8 +607,9 @@ bool plan_lrun(const SppConsts& k, const DevState& d, int K, RunPlan* plan) {
   LrunKernel f = lrun_kernel(lanes, K);
   int fit = 0;
   if (blocks > RUN_MAX_BLOCKS ||
-      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, RUN_SMEM * most) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, f, threads, (size_t)RUN_SMEM * threads) != cudaSuccess) {
+      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * RUN_ROWS_LONG * most) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, f, threads,
+                                                    (size_t)4 * RUN_ROWS_LONG * threads) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -590,7 +628,7 @@ int launch_lrun(const SppConsts& k, const DevState& d, const LyapState& L, const
   attr[0].val.cooperative = 1;
   cfg.gridDim = dim3(plan.blocks);
   cfg.blockDim = dim3(plan.threads);
-  cfg.dynamicSmemBytes = (size_t)RUN_SMEM * plan.threads;
+  cfg.dynamicSmemBytes = (size_t)4 * run_rows(d.cap, k.lanes, 1) * plan.threads;
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;

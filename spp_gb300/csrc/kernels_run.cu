@@ -60,6 +60,9 @@ struct Cold<2> {
  * at unit density, groups of 2 / 4): one lane, one block per SM, N = 65,536:
  * 10.35 / 10.01 and 18.2 / 17.4; two blocks per SM (56 registers), N =
  * 163,840: 14.5 / 15.2 and 24.4 / 25.8; four lanes, N = 16,384: 8.6 / 8.7. */
+/* Long segments (RUN_LONG) are walked 8 at a time instead: 16,384 particles of
+ * the continuous model, 60% of them in flocks with lists of up to 159, 48 -> 41
+ * us per RK4 step. */
 __host__ __device__ constexpr int run_group(int lanes, int per_sm) { return lanes == 1 && per_sm == 1 ? 4 : 2; }
 
 template <int LAW, int KIND>
@@ -86,14 +89,16 @@ __global__ void __launch_bounds__(run_threads(PER_SM), PER_SM) k_run(const __gri
                                                          int nst, int nsteps) {
   constexpr bool BEADLIKE = (KIND == SPP_KIND_BEADS || KIND == SPP_KIND_CHAIN);
   constexpr int GROUP = run_group(LANES, PER_SM);
+  constexpr int BIG = PER_SM == 1 && KIND != SPP_KIND_CHAIN ? 8 : 0;   /* the same for long segments */
   extern __shared__ __align__(16) unsigned char run_smem[];
   __shared__ unsigned fin[2][2];
   __shared__ unsigned s_word;
   const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
-  int32_t* const rows = reinterpret_cast<int32_t*>(run_smem) + tid;                        /* [RUN_ROWS][T] */
+  const int R = run_rows(d.cap, LANES, PER_SM);
+  int32_t* const rows = reinterpret_cast<int32_t*>(run_smem) + tid;                        /* [R][T] */
   unsigned long long* const keycol = reinterpret_cast<unsigned long long*>(run_smem) + tid; /* [LIST_LOCAL][T] */
-  int32_t* const ring = reinterpret_cast<int32_t*>(run_smem + (size_t)RUN_SMEM * T) + tid;  /* [4][T] */
-  Cold<PER_SM> cold(reinterpret_cast<float*>(run_smem + (size_t)(RUN_SMEM + (BEADLIKE ? RING_SMEM : 0)) * T) + tid, T);
+  int32_t* const ring = reinterpret_cast<int32_t*>(run_smem + (size_t)R * 4 * T) + tid;     /* [4][T] */
+  Cold<PER_SM> cold(reinterpret_cast<float*>(run_smem + (size_t)(R * 4 + (BEADLIKE ? RING_SMEM : 0)) * T) + tid, T);
   Ctl* const ctl = d.ctl;
   const int n = d.n;
   const int i = (blockIdx.x * T + tid) / LANES;
@@ -107,8 +112,9 @@ __global__ void __launch_bounds__(run_threads(PER_SM), PER_SM) k_run(const __gri
   float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   uint32_t pid = 0u;
   int q_begin = 0, len = 0;
-  /* the particle and its list from global memory */
-  auto load = [&](bool with_list) {
+  bool wide = false;
+  /* the particle and its list from global memory (all threads call) */
+  auto load_own = [&](bool with_list) {
     if (!inb) return;
     p = d.pos[i];
     pid = d.id[i];
@@ -124,7 +130,7 @@ __global__ void __launch_bounds__(run_threads(PER_SM), PER_SM) k_run(const __gri
       for (int r = 0; r < lane_r; ++r) q_begin += (int)((lc >> (16 * r)) & 0xffffull);
       len = (int)((lc >> (16 * lane_r)) & 0xffffull);
     }
-    const int m = len < RUN_ROWS ? len : RUN_ROWS;
+    const int m = len < R ? len : R;
     for (int q = 0; q < m; q += 4) {
       int v[4];
 #pragma unroll
@@ -141,6 +147,10 @@ __global__ void __launch_bounds__(run_threads(PER_SM), PER_SM) k_run(const __gri
         ring[o * T] = (int32_t)slot;
       }
     }
+  };
+  auto load = [&](bool with_list) {
+    load_own(with_list);
+    wide = __reduce_max_sync(0xffffffffu, (unsigned)len) >= (unsigned)RUN_LONG;
   };
   auto noise = [&](uint32_t at) -> float {
     if (!head || (BEADLIKE && pid < (uint32_t)k.n_beads)) return 0.0f;
@@ -183,13 +193,32 @@ __global__ void __launch_bounds__(run_threads(PER_SM), PER_SM) k_run(const __gri
           rp[o] = make_float4(v.x, v.y, 0.0f, 0.0f);
         }
       }
-      for (int q0 = 0; q0 < len; q0 += GROUP) {
+      int q0 = 0;
+      if (BIG > 0 && wide)
+        for (; q0 + BIG <= len; q0 += BIG) {
+          int jg[BIG > 0 ? BIG : 1];
+          float4 pg[BIG > 0 ? BIG : 1];
+#pragma unroll
+          for (int u = 0; u < BIG; ++u) {
+            const int q = q0 + u;
+            jg[u] = q < R ? rows[q * T] : d.nbr[(size_t)(q_begin + q) * n + i];
+            if (!spp_index_ok(ctl, jg[u], n)) jg[u] = i;
+          }
+#pragma unroll
+          for (int u = 0; u < BIG; ++u) pg[u] = cur[jg[u]];
+#pragma unroll
+          for (int u = 0; u < BIG; ++u) {
+            if (plain) run_pair<LAW, KIND>(k, d, 0, &a, nbi, jg[u], p, pg[u]);
+            else run_pair<LAW, KIND>(k, d, 1, &a, nbi, jg[u], p, pg[u]);
+          }
+        }
+      for (; q0 < len; q0 += GROUP) {
         int jg[GROUP];
         float4 pg[GROUP];
 #pragma unroll
         for (int u = 0; u < GROUP; ++u) {
           const int q = q0 + u;
-          jg[u] = q < len ? (q < RUN_ROWS ? rows[q * T] : d.nbr[(size_t)(q_begin + q) * n + i]) : i;
+          jg[u] = q < len ? (q < R ? rows[q * T] : d.nbr[(size_t)(q_begin + q) * n + i]) : i;
           if (!spp_index_ok(ctl, jg[u], n)) jg[u] = i;
         }
 #pragma unroll
@@ -389,8 +418,8 @@ RunKernel run_kernel(const SppConsts& k, int lanes, int per_sm) {
 
 int run_lanes(const SppConsts& k) { return spp_pair_kind(&k) == SPP_KIND_CHAIN ? 1 : k.lanes; }
 
-size_t run_smem_bytes(const SppConsts& k, int per_sm, int threads) {
-  return (size_t)(RUN_SMEM + (k.model == SPP_MODEL_BEADS ? RING_SMEM : 0) + (per_sm == 2 ? COLD_SMEM : 0)) * threads;
+size_t run_smem_bytes(const SppConsts& k, int rows, int per_sm, int threads) {
+  return (size_t)(4 * rows + (k.model == SPP_MODEL_BEADS ? RING_SMEM : 0) + (per_sm == 2 ? COLD_SMEM : 0)) * threads;
 }
 
 }  // namespace
@@ -414,10 +443,11 @@ bool plan_run(const SppConsts& k, const DevState& d, RunPlan* plan) {
   const int blocks = (int)((total + threads - 1) / threads);
   RunKernel f = run_kernel(k, lanes, per_sm);
   if (!f || blocks > RUN_MAX_BLOCKS) return false;
+  const int most = per_sm == 1 ? RUN_ROWS_LONG : RUN_ROWS;   /* the list may grow */
   int fit = 0;
   if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)run_smem_bytes(k, per_sm, run_threads(per_sm))) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, f, threads, run_smem_bytes(k, per_sm, threads)) != cudaSuccess) {
+                           (int)run_smem_bytes(k, most, per_sm, run_threads(per_sm))) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, f, threads, run_smem_bytes(k, most, per_sm, threads)) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -435,7 +465,7 @@ int launch_run(const SppConsts& k, const DevState& d, const RunPlan& plan, int n
   attr[0].val.cooperative = 1;
   cfg.gridDim = dim3(plan.blocks);
   cfg.blockDim = dim3(plan.threads);
-  cfg.dynamicSmemBytes = run_smem_bytes(k, plan.per_sm, plan.threads);
+  cfg.dynamicSmemBytes = run_smem_bytes(k, run_rows(d.cap, run_lanes(k), plan.per_sm), plan.per_sm, plan.threads);
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;

@@ -9,12 +9,20 @@ namespace {
 
 /* Shared memory per thread: the list build's LIST_LOCAL keys, then the keys
  * of the long-list sort (RUN_SORT_MAX per warp); between rebuilds the same
- * bytes hold the first RUN_ROWS entries of the thread's neighbour segment
- * (later entries are read from global memory). */
+ * bytes hold the first run_rows() entries of the thread's neighbour segment
+ * (later entries are read from global memory): 32 of them, or 64 where the
+ * list capacity (grown by flocks) says that segments run past 32 and one
+ * block per SM leaves the room. */
 constexpr int RUN_SORT_MAX = 512;
 constexpr int RUN_SMEM = RUN_SORT_MAX * 8 / 32;
 static_assert(RUN_SMEM >= LIST_LOCAL * 8, "the build's keys");
-constexpr int RUN_ROWS = RUN_SMEM / 4;
+constexpr int RUN_ROWS = RUN_SMEM / 4, RUN_ROWS_LONG = 64;
+__host__ __device__ inline int run_rows(int cap, int lanes, int per_sm) {
+  return per_sm == 1 && cap > 3 * lanes * RUN_ROWS / 4 ? RUN_ROWS_LONG : RUN_ROWS;
+}
+/* Segments from this length on (the longest of a warp) are walked with more
+ * neighbours in flight. */
+constexpr int RUN_LONG = 12;
 
 /* A queued list (longer than LIST_TAIL) put in order by the calling warp, as
  * sort_queued_list (spp_list.cuh) does, by a bitonic network over keys in
