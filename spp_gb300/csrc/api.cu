@@ -964,7 +964,7 @@ int spp_create(const SppParams* p, SppSystem** out) {
   }
   cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMemset(d.ctl, 0, sizeof(Ctl));
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.ctl, 0, sizeof(Ctl), s->stream);
   if (e != cudaSuccess) {
     free_dev(s);
     delete s;
@@ -1382,8 +1382,9 @@ int spp_lyap_set_vectors(SppSystem* s, const float* v, int K) {
   if (!s || !v) return fail(SPP_ERR_INVALID, "NULL argument");
   if (!s->lyap_on || K != s->lyap.K) return fail(SPP_ERR_INVALID, "spp_lyap_init with this K first");
   CUDA_TRY(cudaStreamSynchronize(s->stream));
-  CUDA_TRY(cudaMemcpy(s->lyap.t0, v, sizeof(float) * (size_t)K * 3 * s->p.n, cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemset(s->lyap.log_stretch, 0, sizeof(double) * SPP_LYAP_MAX));
+  CUDA_TRY(cudaMemcpyAsync(s->lyap.t0, v, sizeof(float) * (size_t)K * 3 * s->p.n, cudaMemcpyHostToDevice, s->stream));
+  CUDA_TRY(cudaMemsetAsync(s->lyap.log_stretch, 0, sizeof(double) * SPP_LYAP_MAX, s->stream));
+  CUDA_TRY(cudaStreamSynchronize(s->stream));
   s->lyap_steps = 0;
   return SPP_OK;
 }

@@ -1306,10 +1306,10 @@ int spp_mlp_create(int ensemble, int in_dim, SppMlp** out) {
     e = cudaFuncSetAttribute(k_mlp_fused<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FUSED_SMEM);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_mlp_fused<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FUSED_SMEM);
-  if (e == cudaSuccess) e = cudaMemset(m->master, 0, sizeof(float) * tot);
-  if (e == cudaSuccess) e = cudaMemset(m->w, 0, sizeof(__nv_bfloat16) * tot);
-  if (e == cudaSuccess) e = cudaMemset(m->mom, 0, sizeof(float) * tot);
-  if (e == cudaSuccess) e = cudaMemset(m->vel, 0, sizeof(float) * tot);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->master, 0, sizeof(float) * tot, m->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->w, 0, sizeof(__nv_bfloat16) * tot, m->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->mom, 0, sizeof(float) * tot, m->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->vel, 0, sizeof(float) * tot, m->stream);
   if (e != cudaSuccess) {
     cudaFree(m->master); cudaFree(m->w); cudaFree(m->mom); cudaFree(m->vel); cudaFree(m->grad); cudaFree(m->pub);
     delete m;
