@@ -7,8 +7,10 @@
  * sweep lives in one set of device arrays, indexed by a per-system offset
  * table (particle range, cell range, constants, activity, step count), and
  * each phase of a step is ONE launch over all particles of all systems:
- *   zero counts | k_batch_bin | scan (global) | k_batch_scatter |
- *   k_batch_step | k_batch_finish
+ *   scan of the cell counts (two launches) | k_batch_scatter | k_batch_step |
+ *   k_batch_finish
+ * k_batch_step also counts the particles into the cells of the next step, so
+ * k_batch_bin runs only when the state or the set of active systems is new.
  * Small systems (1k particles) that alone could not fill the GPU share it
  * with the large ones; the step loop is captured in CUDA graphs.  Retired or
  * finished systems stay in place and are copied through without work.
@@ -19,6 +21,7 @@
  * window -- the inputs and targets of the sweep surrogate.
  */
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -33,126 +36,129 @@ __device__ __forceinline__ int act_slot(const DevBatch& b, int t, int* s) {
   return t + b.sact[*s].a_corr;
 }
 
-/* Keys are compact cell indices: a system's D x D row-major grid starts at
- * its a_coff, so the scan runs over the cells of active systems only and a
- * system's cell starts, plus its a_corr, are slots of its own particle range. */
+/* A particle as its neighbours read it: position, and the exact fixed-point
+ * parts of cos and sin (spp_fx_add: |hi| <= 32, |lo| <= 2^21), each pair packed
+ * as hi << 24 | lo + 2^22. */
+constexpr int PACK_BIAS = 1 << 22;
+__device__ __forceinline__ float pack_parts(spp_fx a) {
+  return __int_as_float((int)((uint32_t)a.hi << 24 | (uint32_t)(a.lo + PACK_BIAS)));
+}
+__device__ __forceinline__ spp_fx fx_parts(float v) {
+  spp_fx a = {0, 0};
+  spp_fx_add(&a, v);
+  return a;
+}
+/* Sums of packed parts: the words add up modulo 2^32 and the upper bytes by
+ * themselves, which leaves the sum of the lower parts exact (two additions
+ * per term). */
+struct PackedSum { int32_t words, hi; };
+__device__ __forceinline__ void packed_add(PackedSum* a, float w) {
+  const int v = __float_as_int(w);
+  a->words += v;
+  a->hi += v >> 24;
+}
+__device__ __forceinline__ spp_fx packed_value(PackedSum a, int terms) {
+  return {a.hi, (int32_t)((uint32_t)a.words - ((uint32_t)a.hi << 24) - (uint32_t)terms * (uint32_t)PACK_BIAS)};
+}
+
+/* Counts particle t, at (x, y), into the compact cells of the next step: its
+ * cell (cx | cy << 16) and its place in it.  Keys are compact cell indices: a
+ * system's D x D row-major grid starts at its a_coff, so the scan runs over
+ * the cells of active systems only and a system's cell starts, plus its
+ * a_corr, are slots of its own particle range. */
+__device__ __forceinline__ void count_particle(const DevBatch& b, const BatchSys& S, uint32_t a_coff, int t, float x,
+                                               float y) {
+  const int cx = spp_cell_coord(x, S.k.L, S.k.L2, (int)S.D, SPP_BIN_GEOMETRIC);
+  const int cy = spp_cell_coord(y, S.k.L, S.k.L2, (int)S.D, SPP_BIN_GEOMETRIC);
+  const uint32_t key = a_coff + (uint32_t)cy * S.D + (uint32_t)cx;
+  b.cell[t] = (uint32_t)cx | (uint32_t)cy << 16;
+  b.rank[t] = atomicAdd(&b.cell_count[key], 1u);   /* moved particles rarely share a cell with their warp */
+}
+
 __global__ void __launch_bounds__(SPP_BLOCK) k_batch_bin(DevBatch b) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= b.n_act) return;
   int s;
   const int i = act_slot(b, t, &s);
-  const BatchSys& S = b.sys[s];
-  const float4 p = b.pos[i];
-  const int cx = spp_cell_coord(p.x, S.k.L, S.k.L2, (int)S.D, SPP_BIN_GEOMETRIC);
-  const int cy = spp_cell_coord(p.y, S.k.L, S.k.L2, (int)S.D, SPP_BIN_GEOMETRIC);
-  const uint32_t key = b.sact[s].a_coff + (uint32_t)cy * S.D + (uint32_t)cx;
-  const unsigned mask = __activemask();
-  const unsigned peers = __match_any_sync(mask, key);
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(peers) - 1;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(&b.cell_count[key], (uint32_t)__popc(peers));
-  base = __shfl_sync(peers, base, leader);
-  b.key[t] = key;
-  b.rank[t] = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+  const float2 p = *reinterpret_cast<const float2*>(b.ent + i);
+  count_particle(b, b.sys[s], b.sact[s].a_coff, t, p.x, p.y);
 }
 
-/* Exact fixed-point parts (hi, lo) of a heading's cos and sin, split as the
- * alignment sums split every term (spp_fx_add).  The scatter computes them
- * once per particle and step, so the neighbour loop of the vector-sum rule
- * adds integers only; the sums, being exact, do not depend on the order in
- * which the candidates are visited. */
-__device__ __forceinline__ int4 fx_parts(float c, float s) {
-  spp_fx a = {0, 0}, b = {0, 0};
-  spp_fx_add(&a, c);
-  spp_fx_add(&b, s);
-  return make_int4(a.hi, a.lo, b.hi, b.lo);
-}
-
+/* Into cell order, within each system's range.  A system that has finished
+ * since the compact space was built stays in place.  THETA: the rules that
+ * read headings (all but the vector sum, whose step needs none). */
+template <bool THETA>
 __global__ void __launch_bounds__(SPP_BLOCK) k_batch_scatter(DevBatch b) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= b.n_act) return;
   int s;
   const int i = act_slot(b, t, &s);
-  const uint32_t dst = b.cell_start[b.key[t]] + b.rank[t] + (uint32_t)b.sact[s].a_corr;
-  const float4 p = b.pos[i];
-  b.pos_alt[dst] = p;
-  b.fx_alt[dst] = fx_parts(p.z, p.w);
-  b.theta_alt[dst] = b.theta[i];
-  b.img_alt[dst] = b.img[i];
+  const uint32_t cell = b.cell[t];
+  const SysAct A = b.sact[s];
+  const BatchSys& S = b.sys[s];
+  const uint32_t key = A.a_coff + (cell >> 16) * S.D + (cell & 0xffffu);
+  const uint32_t dst = S.active ? b.cell_start[key] + b.rank[t] + (uint32_t)A.a_corr : (uint32_t)i;
+  b.ent_alt[dst] = b.ent[i];
   b.id_alt[dst] = b.id[i];
+  b.cell_alt[dst] = cell;
+  if (THETA) b.theta_alt[dst] = b.theta[i];
 }
-
-#ifndef SPP_BATCH_UNROLL
-#define SPP_BATCH_UNROLL 2       /* candidates whose loads are issued together */
-#endif
-#ifndef SPP_BATCH_MIN_BLOCKS
-#define SPP_BATCH_MIN_BLOCKS 6   /* resident 256-thread blocks per SM the step kernel is built for */
-#endif
 
 /* Models of the batch step kernel: one rule for all systems of the batch
  * (the common case), or any mix (runtime dispatch per system). */
 constexpr int BATCH_MIXED = -1;
 
-/* One candidate j of particle i (cell-ordered slot i, position p); q and f
- * are candidate j's position record and fixed-point heading parts. */
+/* The sums a particle receives. */
+struct BatchAcc {
+  PackedSum cx, cy;       /* headings of the aligning neighbours */
+  SppAcc a;               /* count, angles (ax, ay: the push terms) */
+};
+
+/* One candidate j of particle i (cell-ordered slots), its entry q. */
 template <int MODEL>
 __device__ __forceinline__ void visit(const DevBatch& b, const SppConsts& k, int interior, float4 p, int i,
-                                      uint32_t j, float4 q, int4 f, SppAcc* a) {
+                                      uint32_t j, float4 q, BatchAcc* acc) {
   const int model = MODEL == BATCH_MIXED ? k.model : MODEL;
-  if (model == SPP_MODEL_VICSEK) {
-    float dx, dy, d2;
-    if (interior) {
-      dx = p.x - q.x;
-      dy = p.y - q.y;
-      d2 = fmaf(dx, dx, dy * dy);
-    } else {
-      d2 = spp_sep(&k, p.x, p.y, q.x, q.y, &dx, &dy);
-    }
-    if (d2 < k.ral2) {
-      a->ax.hi += f.x;
-      a->ax.lo += f.y;
-      a->ay.hi += f.z;
-      a->ay.lo += f.w;
-      a->cnt += 1;
-    }
+  float dx, dy, d2;
+  if (interior) {
+    dx = p.x - q.x;
+    dy = p.y - q.y;
+    d2 = fmaf(dx, dx, dy * dy);
   } else {
-    const float thj = model == SPP_MODEL_VICSEK_REF_ANGLE ? b.theta_alt[j] : 0.0f;
-    spp_pair_vicsek(&k, a, p.x, p.y, q.x, q.y, q.z, q.w, thj, (int)j == i);
+    d2 = spp_sep(&k, p.x, p.y, q.x, q.y, &dx, &dy);
   }
+  if (!(d2 < k.ral2)) return;
+  if (model != SPP_MODEL_VICSEK && (int)j == i) return;   /* the vector sum counts the particle itself */
+  acc->a.cnt += 1;
+  if (model == SPP_MODEL_VICSEK_REF_ANGLE) {
+    spp_fx_add_guarded(&acc->a.at, b.theta_alt[j], &acc->a.ovf);
+    return;
+  }
+  packed_add(&acc->cx, q.z);
+  packed_add(&acc->cy, q.w);
+  if (model == SPP_MODEL_VICSEK_REF_VECTOR && d2 < k.rpush2 && d2 > 0.0f) spp_push_vicsek(&k, &acc->a, dx, dy, d2);
 }
 
 /* Walks a lane's candidate sequence t = 0 .. T-1 (T the warp's longest):
  * segments of lengths l0, l01 - l0, lt - l01 starting at slots m0, m1 + l0,
- * m2 + l01; SPP_BATCH_UNROLL candidates per trip with their loads first. */
-template <int MODEL>
+ * m2 + l01; UNROLL candidates per trip with their loads first. */
+template <int MODEL, int UNROLL>
 __device__ __forceinline__ void walk(const DevBatch& b, const SppConsts& k, int interior, float4 p, int i, int T,
                                      int lt, int l0, int l01, uint32_t m0, uint32_t m1, uint32_t m2,
-                                     SppAcc* a) {
-  const int vec = MODEL == BATCH_MIXED ? (k.model == SPP_MODEL_VICSEK) : (MODEL == SPP_MODEL_VICSEK);
-  for (int t0 = 0; t0 < T; t0 += SPP_BATCH_UNROLL) {
-    float4 q[SPP_BATCH_UNROLL];
-    int4 f[SPP_BATCH_UNROLL];
-    uint32_t j[SPP_BATCH_UNROLL];
+                                     BatchAcc* acc) {
+  for (int t0 = 0; t0 < T; t0 += UNROLL) {
+    float4 q[UNROLL];
+    uint32_t j[UNROLL];
 #pragma unroll
-    for (int u = 0; u < SPP_BATCH_UNROLL; ++u) {
+    for (int u = 0; u < UNROLL; ++u) {
       const int t = t0 + u;
       j[u] = (uint32_t)t + (t < l0 ? m0 : (t < l01 ? m1 : m2));
       q[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      f[u] = make_int4(0, 0, 0, 0);
-      if (t < lt) {
-        if (MODEL == SPP_MODEL_VICSEK) {  /* the vector rule needs the position only */
-          const float2 xy = __ldg(reinterpret_cast<const float2*>(b.pos_alt + j[u]));
-          q[u] = make_float4(xy.x, xy.y, 0.0f, 0.0f);
-        } else {
-          q[u] = __ldg(b.pos_alt + j[u]);
-        }
-        if (vec) f[u] = __ldg(b.fx_alt + j[u]);
-      }
+      if (t < lt) q[u] = __ldg(b.ent_alt + j[u]);
     }
 #pragma unroll
-    for (int u = 0; u < SPP_BATCH_UNROLL; ++u)
-      if (t0 + u < lt) visit<MODEL>(b, k, interior, p, i, j[u], q[u], f[u], a);
+    for (int u = 0; u < UNROLL; ++u)
+      if (t0 + u < lt) visit<MODEL>(b, k, interior, p, i, j[u], q[u], acc);
   }
 }
 
@@ -181,7 +187,7 @@ __device__ __forceinline__ void segments(const DevBatch& b, const BatchSys* S, S
     lo[r] = hi[r] = 0;
     if (!none) {
       lo[r] = b.cell_start[row + (uint32_t)ca] + (uint32_t)A.a_corr;
-      hi[r] = b.cell_start[row + (uint32_t)cb] + b.cell_count[row + (uint32_t)cb] + (uint32_t)A.a_corr;
+      hi[r] = b.cell_start[row + (uint32_t)cb + 1u] + (uint32_t)A.a_corr;   /* one start past the last cell */
     }
   }
   *m0 = lo[0];
@@ -204,30 +210,40 @@ __device__ __forceinline__ void segments(const DevBatch& b, const BatchSys* S, S
  * a row (a particle in the first or last column) is walked in a second pass,
  * entered only by warps that have such a lane.  A warp whose particles all
  * sit in interior cells (no wrap in any candidate) takes plain differences
- * instead of minimum images: for such pairs the two are the same number. */
-template <int MODEL>
-__global__ void __launch_bounds__(SPP_BLOCK, SPP_BATCH_MIN_BLOCKS) k_batch_step(DevBatch b) {
+ * instead of minimum images: for such pairs the two are the same number.
+ *
+ * Measured, full 512-point sweep (7.4M particles, us per batched step): 888 ->
+ * 603 early, 815 -> 539 after 1,500 steps.  Of that, one 16-byte entry per
+ * candidate instead of 24 bytes, and 56 instead of 92 bytes per particle
+ * moved by the scatter (headings and box crossings no longer travel); the
+ * binning pass folded in here (20 bytes read again, a launch); a two-launch
+ * scan that clears the counts, 25 us instead of 90 (k_scan_counts); the
+ * bookkeeping beside the scan.  What bounds it: issue (about 1,150
+ * instructions per warp, 62% of issue slots) and the walk's loads. */
+template <int MODEL, int UNROLL, int MIN_BLOCKS>
+__global__ void __launch_bounds__(SPP_BLOCK, MIN_BLOCKS) k_batch_step(DevBatch b) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  long long ux = 0, uy = 0;
+  int hx = 0, lx = 0, hy = 0, ly = 0;
   int s = -1, i = -1;
   int active = 0;
   const BatchSys* S = nullptr;
   SysAct A = {0u, 0};
   float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  int cx = 0, cy = 0, interior = 1, edge = 0;
+  uint32_t m0 = 0, m1 = 0, m2 = 0;
+  int l0 = 0, l01 = 0, lt = 0;
   if (t < b.n_act) {
     i = act_slot(b, t, &s);
     S = &b.sys[s];
     A = b.sact[s];
     active = (int)S->active;
-    p = b.pos_alt[i];
+    p = b.ent_alt[i];
   }
-  int cx = 0, cy = 0, interior = 1, edge = 0;
-  uint32_t m0 = 0, m1 = 0, m2 = 0;
-  int l0 = 0, l01 = 0, lt = 0;
   if (active) {
     const int D = (int)S->D;
-    cx = spp_cell_coord(p.x, S->k.L, S->k.L2, D, SPP_BIN_GEOMETRIC);
-    cy = spp_cell_coord(p.y, S->k.L, S->k.L2, D, SPP_BIN_GEOMETRIC);
+    const uint32_t cell = b.cell_alt[i];
+    cx = (int)(cell & 0xffffu);
+    cy = (int)(cell >> 16);
     /* |dx|, |dy| < 2 cell widths <= L for D >= 4: no image is ever nearer */
     interior = (D >= 4 && cx >= 1 && cx <= D - 2 && cy >= 1 && cy <= D - 2);
     edge = (cx == 0 || cx == D - 1);
@@ -236,66 +252,61 @@ __global__ void __launch_bounds__(SPP_BLOCK, SPP_BATCH_MIN_BLOCKS) k_batch_step(
   const int all_interior = __all_sync(0xffffffffu, interior);
   const int any_edge = __any_sync(0xffffffffu, edge);
   const int T = (int)__reduce_max_sync(0xffffffffu, (unsigned)lt);
-  SppAcc a;
-  spp_acc_zero(&a);
-  if (active) walk<MODEL>(b, S->k, all_interior, p, i, T, lt, l0, l01, m0, m1, m2, &a);
+  BatchAcc acc;
+  acc.cx = acc.cy = {0, 0};
+  spp_acc_zero(&acc.a);
+  if (active) walk<MODEL, UNROLL>(b, S->k, all_interior, p, i, T, lt, l0, l01, m0, m1, m2, &acc);
   if (any_edge) {
     lt = 0;
     if (active) segments(b, S, A, cx, cy, 1, &m0, &m1, &m2, &l0, &l01, &lt);
     const int WT = (int)__reduce_max_sync(0xffffffffu, (unsigned)lt);
-    if (active) walk<MODEL>(b, S->k, 0, p, i, WT, lt, l0, l01, m0, m1, m2, &a);
+    if (active) walk<MODEL, UNROLL>(b, S->k, 0, p, i, WT, lt, l0, l01, m0, m1, m2, &acc);
   }
   if (active) {
     const SppConsts& k = S->k;
-    if (a.ovf) atomicOr(&b.ctl->fx_overflow, 1u);
-    const float th0 = b.theta_alt[i];
-    const uint32_t id = b.id_alt[i];
-    const spp_u32x4 r = spp_draw(k.seed, k.system, id, S->steps, SPP_RNG_VICSEK);
-    float x, y, c, sn, t;
-    int gx = 0, gy = 0;
-    spp_vicsek_update(&k, &a, p.x, p.y, th0, p.z, p.w, r.v[0], &x, &y, &t, &c, &sn, &gx, &gy);
-    const int2 g = b.img_alt[i];
-    b.pos[i] = make_float4(x, y, c, sn);
-    b.theta[i] = t;
-    b.img[i] = make_int2(g.x + gx, g.y + gy);
-    b.id[i] = id;
-    spp_fx hx = {0, 0}, hy = {0, 0};
-    spp_fx_add(&hx, c);
-    spp_fx_add(&hy, sn);
-    ux = spp_fx_units(hx);
-    uy = spp_fx_units(hy);
-  } else {
-    if (i >= 0) {  /* finished since the compact space was built: copied through */
-      b.pos[i] = p;
-      b.theta[i] = b.theta_alt[i];
-      b.img[i] = b.img_alt[i];
-      b.id[i] = b.id_alt[i];
+    if (acc.a.ovf) atomicOr(&b.ctl->fx_overflow, 1u);
+    const spp_fx fx = packed_value(acc.cx, acc.a.cnt), fy = packed_value(acc.cy, acc.a.cnt);
+    if (MODEL != SPP_MODEL_VICSEK_REF_ANGLE) {   /* (a mixed batch's angle rule does not read them) */
+      acc.a.ax.hi += fx.hi;
+      acc.a.ax.lo += fx.lo;
+      acc.a.ay.hi += fy.hi;
+      acc.a.ay.lo += fy.lo;
     }
-    s = -1;  /* no contribution */
+    const uint32_t id = b.id_alt[i];
+    float th0 = 0.0f, c0 = 0.0f, s0 = 0.0f;
+    if (MODEL != SPP_MODEL_VICSEK) {
+      th0 = b.theta_alt[i];
+      spp_sincosf(th0, &s0, &c0);   /* as the step before left them */
+    }
+    const spp_u32x4 r = spp_draw(k.seed, k.system, id, S->steps, SPP_RNG_VICSEK);
+    float x, y, c, sn, th;
+    int gx = 0, gy = 0;
+    spp_vicsek_update(&k, &acc.a, p.x, p.y, th0, c0, s0, r.v[0], &x, &y, &th, &c, &sn, &gx, &gy);
+    const spp_fx px = fx_parts(c), py = fx_parts(sn);
+    hx = px.hi; lx = px.lo; hy = py.hi; ly = py.lo;
+    p = make_float4(x, y, pack_parts(px), pack_parts(py));
+    b.ent[i] = p;
+    b.theta[i] = th;
+    b.id[i] = id;
+    if (gx | gy) {   /* box crossings, by particle */
+      int2* const g = b.img + S->p_off + id;
+      *g = make_int2(g->x + gx, g->y + gy);
+    }
   }
-  /* heading sums: one atomic per group of lanes of the same system (a tree
-   * when the whole warp is one system, the common case) */
-  const unsigned peers = __match_any_sync(0xffffffffu, s);
+  if (i >= 0) count_particle(b, *S, A.a_coff, t, p.x, p.y);
+  if (!active) s = -1;  /* no contribution */
+  /* heading sums: one atomic per group of lanes of the same system (|hi| <=
+   * 32 and |lo| <= 2^21, so 32 of them fit a word) */
+  const unsigned peers = __all_sync(0xffffffffu, s == __shfl_sync(0xffffffffu, s, 0)) ? 0xffffffffu
+                                                                                     : __match_any_sync(0xffffffffu, s);
   const int lane = threadIdx.x & 31;
   const int leader = __ffs(peers) - 1;
-  long long sx = ux, sy = uy;
-  if (peers == 0xffffffffu) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sx += __shfl_down_sync(0xffffffffu, sx, o);
-      sy += __shfl_down_sync(0xffffffffu, sy, o);
-    }
-  } else {
-    for (int o = 1; o < 32; ++o) {
-      const int src = (lane + o) & 31;
-      const long long vx = __shfl_sync(0xffffffffu, ux, src);
-      const long long vy = __shfl_sync(0xffffffffu, uy, src);
-      if (lane == leader && ((peers >> src) & 1u)) { sx += vx; sy += vy; }
-    }
-  }
+  const int shx = __reduce_add_sync(peers, hx), slx = __reduce_add_sync(peers, lx);
+  const int shy = __reduce_add_sync(peers, hy), sly = __reduce_add_sync(peers, ly);
   if (lane == leader && s >= 0) {
-    atomicAdd(reinterpret_cast<unsigned long long*>(&b.stats[s].sx), (unsigned long long)sx);
-    atomicAdd(reinterpret_cast<unsigned long long*>(&b.stats[s].sy), (unsigned long long)sy);
+    const spp_fx sx = {shx, slx}, sy = {shy, sly};
+    atomicAdd(reinterpret_cast<unsigned long long*>(&b.stats[s].sx), (unsigned long long)spp_fx_units(sx));
+    atomicAdd(reinterpret_cast<unsigned long long*>(&b.stats[s].sy), (unsigned long long)spp_fx_units(sy));
   }
 }
 
@@ -336,27 +347,40 @@ __global__ void k_batch_flags(DevBatch b) {
   if (s < b.n_sys) b.flags[s] = b.sys[s].active;
 }
 
+/* The smallest uploaded particle with a non-finite value and the smallest
+ * outside its system's box, into Ctl::bad_*. */
+__global__ void k_batch_check(DevBatch b, const float* __restrict__ x, const float* __restrict__ y,
+                              const float* __restrict__ th) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= b.n_total) return;
+  const float xi = x[i], yi = y[i], L = b.sys[b.sys_of[i]].k.L;
+  if (!isfinite(xi) || !isfinite(yi) || !isfinite(th[i])) atomicMin(&b.ctl->bad_nonfinite, (uint32_t)i);
+  else if (xi < -L || xi >= L || yi < -L || yi >= L) atomicMin(&b.ctl->bad_range, (uint32_t)i);
+}
+
 __global__ void k_batch_init(DevBatch b, const float* x, const float* y, const float* th) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= b.n_total) return;
   float s, c;
   spp_sincosf(th[i], &s, &c);
-  b.pos[i] = make_float4(x[i], y[i], c, s);
+  b.ent[i] = make_float4(x[i], y[i], pack_parts(fx_parts(c)), pack_parts(fx_parts(s)));
   b.theta[i] = th[i];
   b.img[i] = make_int2(0, 0);
   b.id[i] = (uint32_t)i - b.sys[b.sys_of[i]].p_off;
 }
 
-__global__ void k_batch_gather(DevBatch b, float* x, float* y, float* th, int2* img) {
+__global__ void k_batch_gather(DevBatch b, float* x, float* y, float* th, int32_t* img_x, int32_t* img_y) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= b.n_total) return;
   const BatchSys& S = b.sys[b.sys_of[i]];
   const uint32_t dst = S.p_off + b.id[i];
-  const float4 p = b.pos[i];
+  const float2 p = *reinterpret_cast<const float2*>(b.ent + i);
   x[dst] = p.x;
   y[dst] = p.y;
   th[dst] = b.theta[i];
-  img[dst] = b.img[i];
+  const int2 g = b.img[i];   /* by particle already */
+  img_x[i] = g.x;
+  img_y[i] = g.y;
 }
 
 __global__ void k_batch_set_active(DevBatch b, const int32_t* idx, int count, uint32_t value) {
@@ -391,8 +415,10 @@ struct SppBatch {
   std::vector<BatchSys> host_sys;
   uint32_t n_keys = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;      /* the forked branch of a captured step */
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   float *stage_x = nullptr, *stage_y = nullptr, *stage_t = nullptr;
-  int2* stage_img = nullptr;
+  int32_t *stage_ix = nullptr, *stage_iy = nullptr;
   std::vector<std::pair<int, cudaGraphExec_t>> graphs;
   std::vector<cudaGraph_t> graph_defs;
   int64_t launches = 0;
@@ -400,6 +426,7 @@ struct SppBatch {
   int model = -1;  /* the one model of all systems, or -1 for a mix */
   std::vector<uint32_t> act_flags;  /* the active set the compact launch space was built for */
   bool act_valid = false;
+  bool counted = false;             /* cell_count, cell and rank are those of the current state */
 };
 
 namespace {
@@ -421,31 +448,53 @@ void batch_free(SppBatch* b) {
   b->graphs.clear();
   b->graph_defs.clear();
   DevBatch& d = b->d;
-  void* ptrs[] = {d.sys, d.stats, d.sys_of, d.pos, d.pos_alt, d.theta, d.theta_alt, d.img,
-                  d.img_alt, d.id, d.id_alt, d.key, d.rank, d.cell_count, d.cell_start, d.fx_alt,
-                  d.scan_tmp, d.ctl, d.act_sys, d.sact, d.flags, b->stage_x, b->stage_y, b->stage_t,
-                  b->stage_img};
+  void* ptrs[] = {d.sys, d.stats, d.sys_of, d.ent, d.ent_alt, d.theta, d.theta_alt, d.img, d.id, d.id_alt,
+                  d.cell, d.cell_alt, d.rank, d.cell_count, d.cell_start, d.scan_tmp, d.ctl, d.act_sys, d.sact,
+                  d.flags, b->stage_x, b->stage_y, b->stage_t, b->stage_ix, b->stage_iy};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   memset(&b->d, 0, sizeof(b->d));
   if (b->stream) cudaStreamDestroy(b->stream);
-  b->stream = nullptr;
+  if (b->side) cudaStreamDestroy(b->side);
+  if (b->ev_fork) cudaEventDestroy(b->ev_fork);
+  if (b->ev_join) cudaEventDestroy(b->ev_join);
+  b->stream = b->side = nullptr;
+  b->ev_fork = b->ev_join = nullptr;
 }
 
-int enqueue_batch_step(SppBatch* b, cudaStream_t st) {
+/* Shapes of the step kernel <rule, candidates in flight, blocks per SM>.
+ * Measured on one GB300 (us per batched step; <., 4, 5> / <., 2, 8>): vector
+ * sum, 834k particles 109 / 115 and 186 / 220 with dense flocks; 1.8M 198 / 193
+ * and 281 / 298; 3.6M 346 / 322 and 396 / 391; 7.4M 670 / 602 and 748 / 699.
+ * Small batches wait on their longest walks, large ones want the warps.
+ * Angles: 8 blocks at every size (834k 78 / 77, 7.4M 612 / 560); the push's
+ * registers spill at 8 (834k: 330 at six, 304 at five). */
+constexpr int BATCH_LARGE = 3000000;
+
+/* One step, captured on st.  The per-system bookkeeping (k_batch_finish) runs
+ * beside the next step's scan: it forks off after the step kernel and is
+ * joined before the scatter, the first to read its results (`forked`: a
+ * branch of the step before is open). */
+int enqueue_batch_step(SppBatch* b, cudaStream_t st, bool forked) {
   const DevBatch& d = b->d;
-  BCUDA(cudaMemsetAsync(d.cell_count, 0, sizeof(uint32_t) * (size_t)d.n_act_keys, st));
   const int nb = nblocks(d.n_act);
-  k_batch_bin<<<nb, SPP_BLOCK, 0, st>>>(d);
-  launch_scan_u32(d.cell_count, (uint32_t)d.n_act_keys, d.scan_tmp, d.cell_start, st, nullptr);
-  k_batch_scatter<<<nb, SPP_BLOCK, 0, st>>>(d);
+  launch_scan_counts(d.cell_count, (uint32_t)d.n_act_keys, d.scan_tmp, d.cell_start, st);
+  if (forked) BCUDA(cudaStreamWaitEvent(st, b->ev_join, 0));
+  if (b->model == SPP_MODEL_VICSEK) k_batch_scatter<false><<<nb, SPP_BLOCK, 0, st>>>(d);
+  else k_batch_scatter<true><<<nb, SPP_BLOCK, 0, st>>>(d);
   switch (b->model) {
-    case SPP_MODEL_VICSEK: k_batch_step<SPP_MODEL_VICSEK><<<nb, SPP_BLOCK, 0, st>>>(d); break;
-    case SPP_MODEL_VICSEK_REF_ANGLE: k_batch_step<SPP_MODEL_VICSEK_REF_ANGLE><<<nb, SPP_BLOCK, 0, st>>>(d); break;
-    case SPP_MODEL_VICSEK_REF_VECTOR: k_batch_step<SPP_MODEL_VICSEK_REF_VECTOR><<<nb, SPP_BLOCK, 0, st>>>(d); break;
-    default: k_batch_step<BATCH_MIXED><<<nb, SPP_BLOCK, 0, st>>>(d); break;
+    case SPP_MODEL_VICSEK:
+      if (d.n_act >= BATCH_LARGE) k_batch_step<SPP_MODEL_VICSEK, 2, 8><<<nb, SPP_BLOCK, 0, st>>>(d);
+      else k_batch_step<SPP_MODEL_VICSEK, 4, 5><<<nb, SPP_BLOCK, 0, st>>>(d);
+      break;
+    case SPP_MODEL_VICSEK_REF_ANGLE: k_batch_step<SPP_MODEL_VICSEK_REF_ANGLE, 2, 8><<<nb, SPP_BLOCK, 0, st>>>(d); break;
+    case SPP_MODEL_VICSEK_REF_VECTOR: k_batch_step<SPP_MODEL_VICSEK_REF_VECTOR, 4, 5><<<nb, SPP_BLOCK, 0, st>>>(d); break;
+    default: k_batch_step<BATCH_MIXED, 4, 5><<<nb, SPP_BLOCK, 0, st>>>(d); break;
   }
-  k_batch_finish<<<nblocks(d.n_sys), SPP_BLOCK, 0, st>>>(d);
+  BCUDA(cudaEventRecord(b->ev_fork, st));
+  BCUDA(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
+  k_batch_finish<<<(d.n_sys + 31) / 32, 32, 0, b->side>>>(d);
+  BCUDA(cudaEventRecord(b->ev_join, b->side));
   BCUDA(cudaGetLastError());
   return SPP_OK;
 }
@@ -494,6 +543,7 @@ int batch_refresh_active(SppBatch* b) {
   d.n_act_keys = (int)a_coff;
   b->act_flags = flags;
   b->act_valid = true;
+  b->counted = false;
   return SPP_OK;
 }
 
@@ -503,7 +553,9 @@ int batch_graph(SppBatch* b, int nsteps, cudaGraphExec_t* out) {
   cudaGraph_t graph = nullptr;
   BCUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   int rc = SPP_OK;
-  for (int i = 0; i < nsteps && rc == SPP_OK; ++i) rc = enqueue_batch_step(b, b->stream);
+  for (int i = 0; i < nsteps && rc == SPP_OK; ++i) rc = enqueue_batch_step(b, b->stream, i > 0);
+  if (rc == SPP_OK && nsteps > 0 && cudaStreamWaitEvent(b->stream, b->ev_join, 0) != cudaSuccess)
+    rc = bfail(SPP_ERR_CUDA, "capture: join");
   cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
   if (rc != SPP_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
   if (e != cudaSuccess) return bfail(SPP_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
@@ -521,13 +573,20 @@ int batch_graph(SppBatch* b, int nsteps, cudaGraphExec_t* out) {
 
 int batch_step_enqueue(SppBatch* b, int nsteps) {
   if (b->d.n_act == 0) return SPP_OK;  /* nothing active */
+  if (nsteps > 0 && !b->counted) {
+    BCUDA(cudaMemsetAsync(b->d.cell_count, 0, sizeof(uint32_t) * (size_t)b->d.n_act_keys, b->stream));
+    k_batch_bin<<<nblocks(b->d.n_act), SPP_BLOCK, 0, b->stream>>>(b->d);
+    BCUDA(cudaGetLastError());
+    b->launches += 1;
+    b->counted = true;
+  }
   while (nsteps > 0) {
     int chunk = nsteps >= BATCH_GRAPH_CHUNK ? BATCH_GRAPH_CHUNK : nsteps;
     cudaGraphExec_t exec;
     int rc = batch_graph(b, chunk, &exec);
     if (rc != SPP_OK) return rc;
     BCUDA(cudaGraphLaunch(exec, b->stream));
-    b->launches += (int64_t)chunk * 7;
+    b->launches += (int64_t)chunk * 5;
     nsteps -= chunk;
   }
   return SPP_OK;
@@ -590,19 +649,18 @@ int spp_batch_create(const SppParams* systems, int n_systems, SppBatch** out) {
   rc = rc ? rc : balloc(&d.sys, (size_t)n_systems);
   rc = rc ? rc : balloc(&d.stats, (size_t)n_systems);
   rc = rc ? rc : balloc(&d.sys_of, n);
-  rc = rc ? rc : balloc(&d.pos, n);
-  rc = rc ? rc : balloc(&d.pos_alt, n);
+  rc = rc ? rc : balloc(&d.ent, n);
+  rc = rc ? rc : balloc(&d.ent_alt, n);
   rc = rc ? rc : balloc(&d.theta, n);
-  rc = rc ? rc : balloc(&d.theta_alt, n);
+  rc = rc ? rc : balloc(&d.theta_alt, b->model == SPP_MODEL_VICSEK ? 1 : n);
   rc = rc ? rc : balloc(&d.img, n);
-  rc = rc ? rc : balloc(&d.img_alt, n);
-  rc = rc ? rc : balloc(&d.fx_alt, n);
   rc = rc ? rc : balloc(&d.id, n);
   rc = rc ? rc : balloc(&d.id_alt, n);
-  rc = rc ? rc : balloc(&d.key, n);
+  rc = rc ? rc : balloc(&d.cell, n);
+  rc = rc ? rc : balloc(&d.cell_alt, n);
   rc = rc ? rc : balloc(&d.rank, n);
   rc = rc ? rc : balloc(&d.cell_count, (size_t)c_off);
-  rc = rc ? rc : balloc(&d.cell_start, (size_t)c_off);
+  rc = rc ? rc : balloc(&d.cell_start, (size_t)c_off + 1);
   rc = rc ? rc : balloc(&d.scan_tmp, ((size_t)c_off + 4095) / 4096 + 1);
   rc = rc ? rc : balloc(&d.ctl, 1);
   rc = rc ? rc : balloc(&d.act_sys, n);
@@ -611,7 +669,8 @@ int spp_batch_create(const SppParams* systems, int n_systems, SppBatch** out) {
   rc = rc ? rc : balloc(&b->stage_x, n);
   rc = rc ? rc : balloc(&b->stage_y, n);
   rc = rc ? rc : balloc(&b->stage_t, n);
-  rc = rc ? rc : balloc(&b->stage_img, n);
+  rc = rc ? rc : balloc(&b->stage_ix, n);
+  rc = rc ? rc : balloc(&b->stage_iy, n);
   if (rc != SPP_OK) {
     batch_free(b);
     delete b;
@@ -621,10 +680,17 @@ int spp_batch_create(const SppParams* systems, int n_systems, SppBatch** out) {
   for (int s = 0; s < n_systems; ++s)
     for (uint32_t q = 0; q < b->host_sys[s].n; ++q) sys_of[b->host_sys[s].p_off + q] = (uint32_t)s;
   cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMemcpy(d.sys, b->host_sys.data(), sizeof(BatchSys) * n_systems, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(d.sys_of, sys_of.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(d.stats, 0, sizeof(BatchStats) * n_systems);
-  if (e == cudaSuccess) e = cudaMemset(d.ctl, 0, sizeof(Ctl));
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
+  /* on the batch's own stream, which does not wait for the legacy one */
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(d.sys, b->host_sys.data(), sizeof(BatchSys) * n_systems, cudaMemcpyHostToDevice, b->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(d.sys_of, sys_of.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, b->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.stats, 0, sizeof(BatchStats) * n_systems, b->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.ctl, 0, sizeof(Ctl), b->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);   /* sys_of goes out of scope */
   if (e != cudaSuccess) {
     batch_free(b);
     delete b;
@@ -659,20 +725,22 @@ int spp_batch_set_windows(SppBatch* b, int window_steps, int stationary_from, in
 int spp_batch_upload(SppBatch* b, const float* x, const float* y, const float* theta, int total_n) {
   if (!b || !x || !y || !theta) return bfail(SPP_ERR_INVALID, "NULL argument");
   if (total_n != b->d.n_total) return bfail(SPP_ERR_INVALID, "total_n differs from the batch size");
-  for (const BatchSys& S : b->host_sys) {
-    const float L = S.k.L;
-    for (uint32_t q = 0; q < S.n; ++q) {
-      const uint32_t i = S.p_off + q;
-      if (!std::isfinite(x[i]) || !std::isfinite(y[i]) || !std::isfinite(theta[i]))
-        return bfail(SPP_ERR_NUMERIC, "non-finite input at particle " + std::to_string(i));
-      if (x[i] < -L || x[i] >= L || y[i] < -L || y[i] >= L)
-        return bfail(SPP_ERR_INVALID, "position outside its system's box at particle " + std::to_string(i));
-    }
-  }
-  size_t bytes = sizeof(float) * (size_t)total_n;
+  const size_t bytes = sizeof(float) * (size_t)total_n;
   BCUDA(cudaMemcpyAsync(b->stage_x, x, bytes, cudaMemcpyHostToDevice, b->stream));
   BCUDA(cudaMemcpyAsync(b->stage_y, y, bytes, cudaMemcpyHostToDevice, b->stream));
   BCUDA(cudaMemcpyAsync(b->stage_t, theta, bytes, cudaMemcpyHostToDevice, b->stream));
+  /* checked on the device, before anything of the batch's state changes (the
+   * host took 2 ms per million particles) */
+  uint32_t bad[2] = {0xffffffffu, 0xffffffffu};
+  static_assert(offsetof(Ctl, bad_range) == offsetof(Ctl, bad_nonfinite) + sizeof(uint32_t), "read together");
+  BCUDA(cudaMemcpyAsync(&b->d.ctl->bad_nonfinite, bad, sizeof(bad), cudaMemcpyHostToDevice, b->stream));
+  k_batch_check<<<nblocks(total_n), SPP_BLOCK, 0, b->stream>>>(b->d, b->stage_x, b->stage_y, b->stage_t);
+  b->launches += 1;
+  BCUDA(cudaMemcpyAsync(bad, &b->d.ctl->bad_nonfinite, sizeof(bad), cudaMemcpyDeviceToHost, b->stream));
+  BCUDA(cudaStreamSynchronize(b->stream));
+  if (bad[0] < bad[1]) return bfail(SPP_ERR_NUMERIC, "non-finite input at particle " + std::to_string(bad[0]));
+  if (bad[1] != 0xffffffffu)
+    return bfail(SPP_ERR_INVALID, "position outside its system's box at particle " + std::to_string(bad[1]));
   /* reset per-system counters and statistics */
   for (auto& S : b->host_sys) { S.active = 1u; S.steps = 0u; }
   BCUDA(cudaMemcpyAsync(b->d.sys, b->host_sys.data(), sizeof(BatchSys) * b->host_sys.size(),
@@ -683,6 +751,7 @@ int spp_batch_upload(SppBatch* b, const float* x, const float* y, const float* t
   b->launches += 1;
   BCUDA(cudaStreamSynchronize(b->stream));
   b->uploaded = true;
+  b->counted = false;
   return SPP_OK;
 }
 
@@ -762,23 +831,15 @@ int spp_batch_download(SppBatch* b, float* x, float* y, float* theta, int32_t* i
                        int32_t* img_y, int total_n) {
   if (!b || !x || !y || !theta || total_n != b->d.n_total) return bfail(SPP_ERR_INVALID, "bad arguments");
   k_batch_gather<<<nblocks(total_n), SPP_BLOCK, 0, b->stream>>>(b->d, b->stage_x, b->stage_y,
-                                                                  b->stage_t, b->stage_img);
+                                                                  b->stage_t, b->stage_ix, b->stage_iy);
   b->launches += 1;
   size_t bytes = sizeof(float) * (size_t)total_n;
   BCUDA(cudaMemcpyAsync(x, b->stage_x, bytes, cudaMemcpyDeviceToHost, b->stream));
   BCUDA(cudaMemcpyAsync(y, b->stage_y, bytes, cudaMemcpyDeviceToHost, b->stream));
   BCUDA(cudaMemcpyAsync(theta, b->stage_t, bytes, cudaMemcpyDeviceToHost, b->stream));
-  std::vector<int2> img;
-  if (img_x || img_y) {
-    img.resize((size_t)total_n);
-    BCUDA(cudaMemcpyAsync(img.data(), b->stage_img, sizeof(int2) * (size_t)total_n,
-                          cudaMemcpyDeviceToHost, b->stream));
-  }
+  if (img_x) BCUDA(cudaMemcpyAsync(img_x, b->stage_ix, bytes, cudaMemcpyDeviceToHost, b->stream));
+  if (img_y) BCUDA(cudaMemcpyAsync(img_y, b->stage_iy, bytes, cudaMemcpyDeviceToHost, b->stream));
   BCUDA(cudaStreamSynchronize(b->stream));
-  for (int i = 0; i < (int)img.size(); ++i) {
-    if (img_x) img_x[i] = img[i].x;
-    if (img_y) img_y[i] = img[i].y;
-  }
   return SPP_OK;
 }
 

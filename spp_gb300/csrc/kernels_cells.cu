@@ -107,6 +107,77 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const uint32_t* __r
   }
 }
 
+/* k_scan_apply for launch_scan_counts: takes its offset from the block sums
+ * themselves (the launch of k_scan_top is saved), adds the total as entry n
+ * and clears the counts.  A warp owns 512 consecutive counts, read, cleared
+ * and written 16 bytes per lane: with four words per thread and blocks of
+ * 1,024 the 7 million cells of the full sweep took 80 to 120 us, waves of
+ * blocks waiting at their barriers; this takes 14. */
+constexpr int SCAN_COUNT_THREADS = 256;
+constexpr int SCAN_COUNT_TRIPS = SCAN_TILE / (SCAN_COUNT_THREADS * 4);
+__global__ void __launch_bounds__(SCAN_COUNT_THREADS) k_scan_counts(uint32_t* counts, uint32_t n,
+                                                                    const uint32_t* __restrict__ block_sums,
+                                                                    uint32_t* __restrict__ out) {
+  __shared__ uint32_t warp_total[SCAN_COUNT_THREADS / 32], warp_before[SCAN_COUNT_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t base = blockIdx.x * SCAN_TILE + warp * (SCAN_COUNT_TRIPS * 128) + lane * 4;
+  uint4 v[SCAN_COUNT_TRIPS];
+#pragma unroll
+  for (int q = 0; q < SCAN_COUNT_TRIPS; ++q) {
+    const uint32_t c = base + q * 128;
+    v[q] = make_uint4(0u, 0u, 0u, 0u);
+    if (c + 4 <= n) {
+      v[q] = *reinterpret_cast<const uint4*>(counts + c);
+    } else {   /* the last few */
+      if (c < n) v[q].x = counts[c];
+      if (c + 1 < n) v[q].y = counts[c + 1];
+      if (c + 2 < n) v[q].z = counts[c + 2];
+    }
+  }
+  uint32_t before = 0;
+  for (uint32_t b = threadIdx.x; b < blockIdx.x; b += SCAN_COUNT_THREADS) before += block_sums[b];
+  /* exclusive prefix of each lane's words within the warp's segment */
+  uint32_t e[SCAN_COUNT_TRIPS], carry = 0;
+#pragma unroll
+  for (int q = 0; q < SCAN_COUNT_TRIPS; ++q) {
+    const uint32_t own = (v[q].x + v[q].y) + (v[q].z + v[q].w);
+    uint32_t incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    e[q] = carry + incl - own;
+    carry += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0) {
+    warp_total[warp] = carry;
+    warp_before[warp] = before;
+  }
+  __syncthreads();
+  uint32_t offset = 0;
+#pragma unroll
+  for (int w = 0; w < SCAN_COUNT_THREADS / 32; ++w) offset += warp_before[w] + (w < warp ? warp_total[w] : 0u);
+#pragma unroll
+  for (int q = 0; q < SCAN_COUNT_TRIPS; ++q) {
+    const uint32_t c = base + q * 128;
+    const uint32_t e0 = offset + e[q], e1 = e0 + v[q].x, e2 = e1 + v[q].y, e3 = e2 + v[q].z;
+    if (c + 4 <= n) {
+      *reinterpret_cast<uint4*>(out + c) = make_uint4(e0, e1, e2, e3);
+      *reinterpret_cast<uint4*>(counts + c) = make_uint4(0u, 0u, 0u, 0u);
+      if (c + 4 == n) out[n] = e3 + v[q].w;
+    } else if (c < n) {
+      const uint32_t x[4] = {e0, e1, e2, e3};
+      for (uint32_t k = 0; c + k < n; ++k) {
+        out[c + k] = x[k];
+        counts[c + k] = 0u;
+      }
+      out[n] = c + 1 == n ? e1 : (c + 2 == n ? e2 : e3);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(SPP_BLOCK) k_scatter(DevState d) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.n) return;
@@ -245,6 +316,12 @@ void launch_scan_u32(const uint32_t* in, uint32_t n, uint32_t* block_tmp, uint32
   k_scan_top<<<1, SCAN_THREADS, 0, s>>>(block_tmp, nb);
   k_scan_apply<<<nb, SCAN_THREADS, 0, s>>>(in, n, block_tmp, out);
   if (launches) *launches += 3;
+}
+
+void launch_scan_counts(uint32_t* counts, uint32_t n, uint32_t* block_tmp, uint32_t* out, cudaStream_t s) {
+  const uint32_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+  k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(counts, n, block_tmp);
+  k_scan_counts<<<nb, SCAN_COUNT_THREADS, 0, s>>>(counts, n, block_tmp, out);
 }
 
 uint32_t scan_max_elements() { return (uint32_t)SCAN_TILE * (uint32_t)SCAN_TILE; }

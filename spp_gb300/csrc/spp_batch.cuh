@@ -34,12 +34,12 @@ struct DevBatch {
   BatchSys* sys;
   BatchStats* stats;
   uint32_t* sys_of;       /* particle slot -> system (static: binning stays inside a system's range) */
-  float4 *pos, *pos_alt;
+  float4 *ent, *ent_alt;  /* (x, y, packed cos, packed sin) by slot; the cell-ordered copy */
   float *theta, *theta_alt;
-  int2 *img, *img_alt;
-  int4* fx_alt;           /* fixed-point (cos hi, cos lo, sin hi, sin lo) of the cell-ordered copy */
+  int2* img;              /* box crossings by particle (system range + id) */
   uint32_t *id, *id_alt;  /* particle id within its system */
-  uint32_t *key, *rank;
+  uint32_t *cell, *cell_alt;  /* cell of the next / of this step, cx | cy << 16 */
+  uint32_t* rank;         /* place in the cell of the next step */
   uint32_t *cell_count, *cell_start, *scan_tmp;
   Ctl* ctl;
   /* compact launch space: the particles and cells of the systems that were

@@ -132,6 +132,9 @@ void launch_scan(const DevState& d, cudaStream_t s, int64_t* launches);
  * ceil(n / 4096) entries */
 void launch_scan_u32(const uint32_t* in, uint32_t n, uint32_t* block_tmp, uint32_t* out,
                      cudaStream_t s, int64_t* launches);
+/* the same for a step's cell counts: out has one entry more (the total), and
+ * the counts are cleared as they are read */
+void launch_scan_counts(uint32_t* counts, uint32_t n, uint32_t* block_tmp, uint32_t* out, cudaStream_t s);
 uint32_t scan_max_elements();
 void launch_scatter(const DevState& d, cudaStream_t s, int64_t* launches);
 void launch_build_list(const SppConsts& k, const DevState& d, int with_list, cudaStream_t s,
