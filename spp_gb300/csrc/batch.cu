@@ -114,24 +114,18 @@ struct BatchAcc {
   SppAcc a;               /* count, angles (ax, ay: the push terms) */
 };
 
-/* One candidate j of particle i (cell-ordered slots), its entry q. */
+/* One candidate (entry q, heading thj for the angle rule) at separation
+ * (dx, dy), self: the particle itself. */
 template <int MODEL>
-__device__ __forceinline__ void visit(const DevBatch& b, const SppConsts& k, int interior, float4 p, int i,
-                                      uint32_t j, float4 q, BatchAcc* acc) {
+__device__ __forceinline__ void visit(const SppConsts& k, float dx, float dy, float4 q, const float* thj, bool self,
+                                      BatchAcc* acc) {
   const int model = MODEL == BATCH_MIXED ? k.model : MODEL;
-  float dx, dy, d2;
-  if (interior) {
-    dx = p.x - q.x;
-    dy = p.y - q.y;
-    d2 = fmaf(dx, dx, dy * dy);
-  } else {
-    d2 = spp_sep(&k, p.x, p.y, q.x, q.y, &dx, &dy);
-  }
+  const float d2 = fmaf(dx, dx, dy * dy);
   if (!(d2 < k.ral2)) return;
-  if (model != SPP_MODEL_VICSEK && (int)j == i) return;   /* the vector sum counts the particle itself */
+  if (model != SPP_MODEL_VICSEK && self) return;   /* the vector sum counts the particle itself */
   acc->a.cnt += 1;
   if (model == SPP_MODEL_VICSEK_REF_ANGLE) {
-    spp_fx_add_guarded(&acc->a.at, b.theta_alt[j], &acc->a.ovf);
+    spp_fx_add_guarded(&acc->a.at, *thj, &acc->a.ovf);
     return;
   }
   packed_add(&acc->cx, q.z);
@@ -139,63 +133,42 @@ __device__ __forceinline__ void visit(const DevBatch& b, const SppConsts& k, int
   if (model == SPP_MODEL_VICSEK_REF_VECTOR && d2 < k.rpush2 && d2 > 0.0f) spp_push_vicsek(&k, &acc->a, dx, dy, d2);
 }
 
-/* Walks a lane's candidate sequence t = 0 .. T-1 (T the warp's longest):
- * segments of lengths l0, l01 - l0, lt - l01 starting at slots m0, m1 + l0,
- * m2 + l01; UNROLL candidates per trip with their loads first. */
+/* Walks the n cell-ordered slots from lo on, UNROLL at a time with their
+ * loads first.  (sx, sy): what the minimum image subtracts from every
+ * separation of these cells. */
 template <int MODEL, int UNROLL>
-__device__ __forceinline__ void walk(const DevBatch& b, const SppConsts& k, int interior, float4 p, int i, int T,
-                                     int lt, int l0, int l01, uint32_t m0, uint32_t m1, uint32_t m2,
-                                     BatchAcc* acc) {
-  for (int t0 = 0; t0 < T; t0 += UNROLL) {
+__device__ __forceinline__ void walk(const DevBatch& b, const SppConsts& k, float2 p, float sx, float sy, int i,
+                                     uint32_t lo, int n, BatchAcc* acc) {
+  const float4* e = b.ent_alt + lo;
+  for (int t = 0; t < n; t += UNROLL, e += UNROLL) {
     float4 q[UNROLL];
-    uint32_t j[UNROLL];
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u) {
-      const int t = t0 + u;
-      j[u] = (uint32_t)t + (t < l0 ? m0 : (t < l01 ? m1 : m2));
-      q[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (t < lt) q[u] = __ldg(b.ent_alt + j[u]);
-    }
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u)
-      if (t0 + u < lt) visit<MODEL>(b, k, interior, p, i, j[u], q[u], acc);
+      if (t + u < n) q[u] = __ldg(e + u);
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u)
+      if (t + u < n) {
+        const spp_f2 r = spp_sub2(spp_sub2(spp_f2_make(p.x, p.y), spp_f2_make(q[u].x, q[u].y)), spp_f2_make(sx, sy));
+        const uint32_t j = lo + (uint32_t)(t + u);
+        visit<MODEL>(k, r.x, r.y, q[u], b.theta_alt + j, (int)j == i, acc);
+      }
   }
 }
 
-/* Segments of the candidate sequence of a particle in cell (cx, cy): for each
- * of the rows cy-1, cy, cy+1 the columns [cx-1, cx+1] clipped to the grid
- * (wrap = 0), or the one column the periodic wrap adds (wrap = 1: column D-1
- * for cx = 0, column 0 for cx = D-1, none otherwise). */
-__device__ __forceinline__ void segments(const DevBatch& b, const BatchSys* S, SysAct A, int cx, int cy,
-                                         int wrap, uint32_t* m0, uint32_t* m1, uint32_t* m2, int* l0, int* l01,
-                                         int* lt) {
+/* The slots of the columns ca .. cb of the three rows around cell (., cy) and
+ * the rows' image shifts. */
+__device__ __forceinline__ void segments(const DevBatch& b, const BatchSys* S, SysAct A, int cy, int ca, int cb,
+                                         uint32_t (&lo)[3], int (&len)[3]) {
   const int D = (int)S->D;
-  int ca, cb;
-  if (!wrap) {
-    ca = cx > 0 ? cx - 1 : 0;
-    cb = cx < D - 1 ? cx + 1 : D - 1;
-  } else {
-    ca = cb = cx == 0 ? D - 1 : 0;
-  }
-  const int none = wrap && cx != 0 && cx != D - 1;
-  uint32_t lo[3], hi[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
     int ny = cy + r - 1;
     ny = ny < 0 ? ny + D : (ny >= D ? ny - D : ny);
     const uint32_t row = A.a_coff + (uint32_t)ny * (uint32_t)D;
-    lo[r] = hi[r] = 0;
-    if (!none) {
-      lo[r] = b.cell_start[row + (uint32_t)ca] + (uint32_t)A.a_corr;
-      hi[r] = b.cell_start[row + (uint32_t)cb + 1u] + (uint32_t)A.a_corr;   /* one start past the last cell */
-    }
+    const uint32_t first = b.cell_start[row + (uint32_t)ca];
+    lo[r] = first + (uint32_t)A.a_corr;
+    len[r] = (int)(b.cell_start[row + (uint32_t)cb + 1u] - first);   /* one start past the last cell */
   }
-  *m0 = lo[0];
-  *l0 = (int)(hi[0] - lo[0]);
-  *l01 = *l0 + (int)(hi[1] - lo[1]);
-  *lt = *l01 + (int)(hi[2] - lo[2]);
-  *m1 = lo[1] - (uint32_t)*l0;   /* slot = t + m1 for l0 <= t < l01 (wraps as unsigned) */
-  *m2 = lo[2] - (uint32_t)*l01;
 }
 
 /* One Vicsek step of every active system (VicsekParticle{,2}::Interact/Move,
@@ -204,22 +177,26 @@ __device__ __forceinline__ void segments(const DevBatch& b, const BatchSys* S, S
  *
  * Candidates: the 3x3 cells around a particle are, per grid row, one run of
  * consecutive keys (row-major keys), i.e. one contiguous range of the
- * cell-ordered arrays; a lane walks its three row ranges as one flattened
- * sequence, and the warp runs the longest lane's count, so lanes diverge only
- * in the length of their sequences.  The cell that the periodic wrap adds to
- * a row (a particle in the first or last column) is walked in a second pass,
- * entered only by warps that have such a lane.  A warp whose particles all
- * sit in interior cells (no wrap in any candidate) takes plain differences
- * instead of minimum images: for such pairs the two are the same number.
+ * cell-ordered arrays, walked one row after the other; the column that the
+ * periodic wrap adds (a particle in the first or last column) is three more
+ * ranges.  The minimum image needs no comparison: what it subtracts is the
+ * same number for every candidate of a range, 0 or +-2 L (where the two
+ * differ, which takes a candidate two cells or more away, both separations
+ * are beyond every cutoff, so neither is used).
  *
- * Measured, full 512-point sweep (7.4M particles, us per batched step): 888 ->
- * 603 early, 815 -> 539 after 1,500 steps.  Of that, one 16-byte entry per
- * candidate instead of 24 bytes, and 56 instead of 92 bytes per particle
- * moved by the scatter (headings and box crossings no longer travel); the
- * binning pass folded in here (20 bytes read again, a launch); a two-launch
- * scan that clears the counts, 25 us instead of 90 (k_scan_counts); the
- * bookkeeping beside the scan.  What bounds it: issue (about 1,150
- * instructions per warp, 62% of issue slots) and the walk's loads. */
+ * Measured, full 512-point sweep (7.4M particles, us per batched step over the
+ * first 32 steps / after 300): 771 / 1,126 at first.  One 16-byte entry per
+ * candidate instead of 24 bytes, 56 instead of 92 bytes per particle moved by
+ * the scatter (headings and box crossings no longer travel), the binning pass
+ * folded in here (20 bytes read again, a launch), a two-launch scan that
+ * clears the counts (25 us instead of 90: k_scan_counts) and the bookkeeping
+ * beside the scan: 504 / 822.  Row by row instead of the three rows flattened
+ * into one sequence with comparisons for the image (about 20 instructions a
+ * candidate -> 13): 479 / 674.  What bounds it: issue (78% of the slots), the
+ * walk's loads, and warps that wait for their longest walk (28 of 32 lanes).
+ * Slower: blocks of 64 or 128 threads (less L1 reuse, 634 and 616 against 605
+ * some 200 steps in), a second copy of the walk without the image shift (811:
+ * spills), the rows as a rolled loop (617). */
 template <int MODEL, int UNROLL, int MIN_BLOCKS>
 __global__ void __launch_bounds__(SPP_BLOCK, MIN_BLOCKS) k_batch_step(DevBatch b) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -229,9 +206,9 @@ __global__ void __launch_bounds__(SPP_BLOCK, MIN_BLOCKS) k_batch_step(DevBatch b
   const BatchSys* S = nullptr;
   SysAct A = {0u, 0};
   float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  int cx = 0, cy = 0, interior = 1, edge = 0;
-  uint32_t m0 = 0, m1 = 0, m2 = 0;
-  int l0 = 0, l01 = 0, lt = 0;
+  BatchAcc acc;
+  acc.cx = acc.cy = {0, 0};
+  spp_acc_zero(&acc.a);
   if (t < b.n_act) {
     i = act_slot(b, t, &s);
     S = &b.sys[s];
@@ -240,27 +217,30 @@ __global__ void __launch_bounds__(SPP_BLOCK, MIN_BLOCKS) k_batch_step(DevBatch b
     p = b.ent_alt[i];
   }
   if (active) {
+    const SppConsts& k = S->k;
     const int D = (int)S->D;
     const uint32_t cell = b.cell_alt[i];
-    cx = (int)(cell & 0xffffu);
-    cy = (int)(cell >> 16);
-    /* |dx|, |dy| < 2 cell widths <= L for D >= 4: no image is ever nearer */
-    interior = (D >= 4 && cx >= 1 && cx <= D - 2 && cy >= 1 && cy <= D - 2);
-    edge = (cx == 0 || cx == D - 1);
-    segments(b, S, A, cx, cy, 0, &m0, &m1, &m2, &l0, &l01, &lt);
-  }
-  const int all_interior = __all_sync(0xffffffffu, interior);
-  const int any_edge = __any_sync(0xffffffffu, edge);
-  const int T = (int)__reduce_max_sync(0xffffffffu, (unsigned)lt);
-  BatchAcc acc;
-  acc.cx = acc.cy = {0, 0};
-  spp_acc_zero(&acc.a);
-  if (active) walk<MODEL, UNROLL>(b, S->k, all_interior, p, i, T, lt, l0, l01, m0, m1, m2, &acc);
-  if (any_edge) {
-    lt = 0;
-    if (active) segments(b, S, A, cx, cy, 1, &m0, &m1, &m2, &l0, &l01, &lt);
-    const int WT = (int)__reduce_max_sync(0xffffffffu, (unsigned)lt);
-    if (active) walk<MODEL, UNROLL>(b, S->k, 0, p, i, WT, lt, l0, l01, m0, m1, m2, &acc);
+    const int cx = (int)(cell & 0xffffu), cy = (int)(cell >> 16);
+    const float L2 = k.L2;
+    uint32_t lo[3];
+    int len[3];
+    segments(b, S, A, cy, max(cx - 1, 0), min(cx + 1, D - 1), lo, len);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const float sy = r == 0 && cy == 0 ? -L2 : (r == 2 && cy == D - 1 ? L2 : 0.0f);
+      walk<MODEL, UNROLL>(b, k, make_float2(p.x, p.y), 0.0f, sy, i, lo[r], len[r], &acc);
+    }
+    if (cx == 0 || cx == D - 1) {   /* the column that the periodic wrap adds */
+      const int cw = cx == 0 ? D - 1 : 0;
+      segments(b, S, A, cy, cw, cw, lo, len);
+#pragma unroll 1
+      for (int r = 0; r < 3; ++r) {
+        const float sy = r == 0 && cy == 0 ? -L2 : (r == 2 && cy == D - 1 ? L2 : 0.0f);
+        const uint32_t l = r == 0 ? lo[0] : (r == 1 ? lo[1] : lo[2]);
+        const int n = r == 0 ? len[0] : (r == 1 ? len[1] : len[2]);
+        walk<MODEL, UNROLL < 2 ? UNROLL : 2>(b, k, make_float2(p.x, p.y), cx == 0 ? -L2 : L2, sy, i, l, n, &acc);
+      }
+    }
   }
   if (active) {
     const SppConsts& k = S->k;
@@ -463,13 +443,18 @@ void batch_free(SppBatch* b) {
 }
 
 /* Shapes of the step kernel <rule, candidates in flight, blocks per SM>.
- * Measured on one GB300 (us per batched step; <., 4, 5> / <., 2, 8>): vector
- * sum, 834k particles 109 / 115 and 186 / 220 with dense flocks; 1.8M 198 / 193
- * and 281 / 298; 3.6M 346 / 322 and 396 / 391; 7.4M 670 / 602 and 748 / 699.
+ * Measured on one GB300 (us per batched step over the first 32 steps / after
+ * 300, flocking):
+ *   vector sum   <., 4, 5>        <., 2, 8>
+ *     834k       68 / 148         64 / 154
+ *     1.8M       145 / 239        138 / 227
+ *     7.4M       538 / 722        479 / 672
  * Small batches wait on their longest walks, large ones want the warps.
- * Angles: 8 blocks at every size (834k 78 / 77, 7.4M 612 / 560); the push's
- * registers spill at 8 (834k: 330 at six, 304 at five). */
-constexpr int BATCH_LARGE = 3000000;
+ * Angles: <., 2, 8> 68 / 77 and 525 / 550 (834k, 7.4M), <., 4, 5> 69 / 75 and
+ * 576 / 613.  The push needs registers: <., 1, 5> 105 / 496 and 827 / 1654,
+ * <., 4, 5> 123 / 591 and 956 / 1979, <., 4, 4> 109 / 480 and 905 / 1769,
+ * <., 1, 6> 127 / 637 and 987 / 2358; mixed batches the same order. */
+constexpr int BATCH_LARGE = 1500000;
 
 /* One step, captured on st.  The per-system bookkeeping (k_batch_finish) runs
  * beside the next step's scan: it forks off after the step kernel and is
@@ -488,8 +473,8 @@ int enqueue_batch_step(SppBatch* b, cudaStream_t st, bool forked) {
       else k_batch_step<SPP_MODEL_VICSEK, 4, 5><<<nb, SPP_BLOCK, 0, st>>>(d);
       break;
     case SPP_MODEL_VICSEK_REF_ANGLE: k_batch_step<SPP_MODEL_VICSEK_REF_ANGLE, 2, 8><<<nb, SPP_BLOCK, 0, st>>>(d); break;
-    case SPP_MODEL_VICSEK_REF_VECTOR: k_batch_step<SPP_MODEL_VICSEK_REF_VECTOR, 4, 5><<<nb, SPP_BLOCK, 0, st>>>(d); break;
-    default: k_batch_step<BATCH_MIXED, 4, 5><<<nb, SPP_BLOCK, 0, st>>>(d); break;
+    case SPP_MODEL_VICSEK_REF_VECTOR: k_batch_step<SPP_MODEL_VICSEK_REF_VECTOR, 1, 5><<<nb, SPP_BLOCK, 0, st>>>(d); break;
+    default: k_batch_step<BATCH_MIXED, 1, 5><<<nb, SPP_BLOCK, 0, st>>>(d); break;
   }
   BCUDA(cudaEventRecord(b->ev_fork, st));
   BCUDA(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
