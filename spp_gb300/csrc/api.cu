@@ -4,8 +4,8 @@
  * One SppSystem owns the device buffers of one periodic box and launches on
  * one CUDA stream.  spp_step() replays CUDA graphs of whole steps:
  *   ABP / continuous:  [stage kernel] x stages  ->  IF(rebuild) { zero counts,
- *                      bin_count, scan x3, scatter, build_list }
- *   Vicsek (dt = 1):   zero counts, bin_count, scan x3, scatter, step kernel
+ *                      bin_count, scan x2, scatter, build_list }
+ *   Vicsek (dt = 1):   zero counts, bin_count, scan x2, scatter, step kernel
  * The IF condition is set on the device by the last stage kernel
  * (cudaGraphSetConditional), so a replay of many steps never returns to the
  * host.  This is the GB300 counterpart of Box::Multi_Step (parallel/box.h:
@@ -978,8 +978,8 @@ int spp_create(const SppParams* p, SppSystem** out) {
     if (s->uses_list && !off) plan_run(s->k, d, &s->run);
     if (!s->uses_list && !off && !(sv && sv[0] == '0') && plan_vrun(s->k, d, &s->vrun)) alloc_vrun(s);
   }
-  s->per_rebuild_kernels = 7;   /* bin_count, scan x3, scatter, build_list, sort_long */
-  s->per_step_kernels = s->uses_list ? (s->nstages == 1 ? 2 : s->nstages) : 6;
+  s->per_rebuild_kernels = 6;   /* bin_count, scan x2, scatter, build_list, sort_long */
+  s->per_step_kernels = s->uses_list ? (s->nstages == 1 ? 2 : s->nstages) : 5;
   *out = s;
   return SPP_OK;
 }

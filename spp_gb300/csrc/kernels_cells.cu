@@ -7,9 +7,8 @@
  * half Verlet list per particle, rebuilt every cell_update_period steps.
  * Here:
  *   1. bin_count: one thread per particle computes its cell's Morton key and
- *      takes a slot in that cell with one atomicAdd per group of lanes
- *      sharing the key (__match_any_sync warp aggregation).
- *   2. scan: exclusive prefix sum of the per-key counts (three passes).
+ *      takes a slot in that cell with an atomicAdd.
+ *   2. scan: exclusive prefix sum of the per-key counts (two passes).
  *   3. scatter: every particle's state moves to its cell-ordered slot, so
  *      that spatial neighbours are neighbours in memory (Morton order keeps
  *      2-D tiles of cells contiguous).
@@ -27,6 +26,9 @@
 
 namespace {
 
+/* One atomic per particle: cells hold one or two, so grouping a warp's equal
+ * keys first (__match_any_sync) saved few atomics and took 16.4 us at N =
+ * 1,048,576 against 8.5. */
 __global__ void __launch_bounds__(SPP_BLOCK) k_bin_count(SppConsts k, DevState d) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) d.ctl->long_n = 0u;   /* the long-list queue of this rebuild (k_build_list) */
@@ -35,15 +37,8 @@ __global__ void __launch_bounds__(SPP_BLOCK) k_bin_count(SppConsts k, DevState d
   int cx, cy;
   uint32_t key = cell_key(k, d, p.x, p.y, &cx, &cy);
   if (!spp_index_ok(d.ctl, key, d.n_keys)) key = 0u;
-  unsigned mask = __activemask();
-  unsigned peers = __match_any_sync(mask, key);
-  int lane = threadIdx.x & 31;
-  int leader = __ffs(peers) - 1;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(&d.cell_count[key], (uint32_t)__popc(peers));
-  base = __shfl_sync(peers, base, leader);
   d.key[i] = key;
-  d.rank[i] = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+  d.rank[i] = atomicAdd(&d.cell_count[key], 1u);
 }
 
 /* ---- exclusive scan of cell_count into cell_start ---------------------- */
@@ -69,52 +64,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t* __
   }
 }
 
-/* Exclusive scan of at most SCAN_TILE block sums, in place (one block). */
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_top(uint32_t* sums, uint32_t nb) {
-  uint32_t v[SCAN_PER_THREAD];
-  uint32_t base = threadIdx.x * SCAN_PER_THREAD;
-  uint32_t local = 0;
-#pragma unroll
-  for (int q = 0; q < SCAN_PER_THREAD; ++q) {
-    v[q] = (base + q < nb) ? sums[base + q] : 0u;
-    local += v[q];
-  }
-  uint32_t excl = block_exclusive_scan(local);
-#pragma unroll
-  for (int q = 0; q < SCAN_PER_THREAD; ++q) {
-    if (base + q < nb) sums[base + q] = excl;
-    excl += v[q];
-  }
-}
-
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const uint32_t* __restrict__ in,
-                                                             uint32_t n,
-                                                             const uint32_t* __restrict__ block_offs,
-                                                             uint32_t* __restrict__ out) {
-  uint32_t base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER_THREAD;
-  uint32_t v[SCAN_PER_THREAD];
-  uint32_t local = 0;
-#pragma unroll
-  for (int q = 0; q < SCAN_PER_THREAD; ++q) {
-    v[q] = (base + q < n) ? in[base + q] : 0u;
-    local += v[q];
-  }
-  uint32_t excl = block_exclusive_scan(local) + block_offs[blockIdx.x];
-#pragma unroll
-  for (int q = 0; q < SCAN_PER_THREAD; ++q) {
-    if (base + q < n) out[base + q] = excl;
-    excl += v[q];
-  }
-}
-
-/* k_scan_apply for launch_scan_counts: takes its offset from the block sums
- * themselves (the launch of k_scan_top is saved), adds the total as entry n
- * and clears the counts.  A warp owns 512 consecutive counts, read, cleared
+/* The second pass: a block takes its offset from the sums of the blocks before
+ * it (a million cells have 256; a launch that scans the sums first costs
+ * more).  NEXT also adds the total as entry n and clears the counts for the
+ * next step of a batch.  counts and out start on 16-byte boundaries.  A warp owns 512 consecutive counts, read, cleared
  * and written 16 bytes per lane: with four words per thread and blocks of
  * 1,024 the 7 million cells of the full sweep took 80 to 120 us, waves of
- * blocks waiting at their barriers; this takes 14. */
+ * blocks waiting at their barriers; this takes 14 (a million cells: the whole
+ * scan 12 -> 8 us). */
 constexpr int SCAN_COUNT_THREADS = 256;
 constexpr int SCAN_COUNT_TRIPS = SCAN_TILE / (SCAN_COUNT_THREADS * 4);
+template <bool NEXT>
 __global__ void __launch_bounds__(SCAN_COUNT_THREADS) k_scan_counts(uint32_t* counts, uint32_t n,
                                                                     const uint32_t* __restrict__ block_sums,
                                                                     uint32_t* __restrict__ out) {
@@ -165,15 +125,15 @@ __global__ void __launch_bounds__(SCAN_COUNT_THREADS) k_scan_counts(uint32_t* co
     const uint32_t e0 = offset + e[q], e1 = e0 + v[q].x, e2 = e1 + v[q].y, e3 = e2 + v[q].z;
     if (c + 4 <= n) {
       *reinterpret_cast<uint4*>(out + c) = make_uint4(e0, e1, e2, e3);
-      *reinterpret_cast<uint4*>(counts + c) = make_uint4(0u, 0u, 0u, 0u);
-      if (c + 4 == n) out[n] = e3 + v[q].w;
+      if (NEXT) *reinterpret_cast<uint4*>(counts + c) = make_uint4(0u, 0u, 0u, 0u);
+      if (NEXT && c + 4 == n) out[n] = e3 + v[q].w;
     } else if (c < n) {
       const uint32_t x[4] = {e0, e1, e2, e3};
       for (uint32_t k = 0; c + k < n; ++k) {
         out[c + k] = x[k];
-        counts[c + k] = 0u;
+        if (NEXT) counts[c + k] = 0u;
       }
-      out[n] = c + 1 == n ? e1 : (c + 2 == n ? e2 : e3);
+      if (NEXT) out[n] = c + 1 == n ? e1 : (c + 2 == n ? e2 : e3);
     }
   }
 }
@@ -191,19 +151,25 @@ __global__ void __launch_bounds__(SPP_BLOCK) k_scatter(DevState d) {
   d.id_alt[dst] = d.id[i];
 }
 
-/* Verlet list from the cell-ordered copy (alt), then the copy moves back
+/* Bound by its instruction stream (a thread per particle, about 15 candidates
+ * for 5 neighbours).  At N = 1,048,576, ABP, unit density, 200 steps in: 87.6
+ * us a launch when accepted neighbours were inserted in id order as they came
+ * (each lane its own depth), 61 with them collected and put in order by a
+ * network (build_particle_list); a whole rebuild 134 -> 101.  40 registers
+ * for six blocks per SM; four or five are not faster.
+ * Verlet list from the cell-ordered copy (alt), then the copy moves back
  * into the primary arrays. with_list == 0 only copies (no list).  The copy
  * always completes, even when some list overflows: the overflow only sets
  * the frozen flag, which stops the stage kernels until the host has grown
  * the list and rebuilt it. */
 template <int LANES>
-__global__ void __launch_bounds__(SPP_BLOCK) k_build_list(SppConsts k, DevState d, int with_list) {
-  __shared__ unsigned long long skeys[LIST_LOCAL][SPP_BLOCK];
+__global__ void __launch_bounds__(SPP_BLOCK, 6) k_build_list(SppConsts k, DevState d, int with_list) {
+  __shared__ uint32_t slots[LIST_LOCAL][SPP_BLOCK];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t cnt = 0;
   if (i < d.n) {
     const float4 p = d.pos_alt[i];
-    if (with_list) cnt = build_particle_list<LANES>(k, d, i, p, &skeys[0][threadIdx.x], SPP_BLOCK);
+    if (with_list) cnt = build_particle_list<LANES>(k, d, i, p, &slots[0][threadIdx.x], SPP_BLOCK);
     adopt_sorted_particle(d, i, p);
   }
   if (with_list) note_list_lengths(d, cnt);
@@ -309,19 +275,18 @@ void launch_bin_count(const SppConsts& k, const DevState& d, cudaStream_t s, int
   if (launches) *launches += 1;
 }
 
-void launch_scan_u32(const uint32_t* in, uint32_t n, uint32_t* block_tmp, uint32_t* out,
-                     cudaStream_t s, int64_t* launches) {
-  uint32_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-  k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(in, n, block_tmp);
-  k_scan_top<<<1, SCAN_THREADS, 0, s>>>(block_tmp, nb);
-  k_scan_apply<<<nb, SCAN_THREADS, 0, s>>>(in, n, block_tmp, out);
-  if (launches) *launches += 3;
+void launch_scan_u32(uint32_t* counts, uint32_t n, uint32_t* block_tmp, uint32_t* out, cudaStream_t s,
+                     int64_t* launches) {
+  const uint32_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+  k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(counts, n, block_tmp);
+  k_scan_counts<false><<<nb, SCAN_COUNT_THREADS, 0, s>>>(counts, n, block_tmp, out);
+  if (launches) *launches += 2;
 }
 
 void launch_scan_counts(uint32_t* counts, uint32_t n, uint32_t* block_tmp, uint32_t* out, cudaStream_t s) {
   const uint32_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
   k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(counts, n, block_tmp);
-  k_scan_counts<<<nb, SCAN_COUNT_THREADS, 0, s>>>(counts, n, block_tmp, out);
+  k_scan_counts<true><<<nb, SCAN_COUNT_THREADS, 0, s>>>(counts, n, block_tmp, out);
 }
 
 uint32_t scan_max_elements() { return (uint32_t)SCAN_TILE * (uint32_t)SCAN_TILE; }

@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
   const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
   const int R = run_rows(d.cap, LANES, 1);
   int32_t* const rows = reinterpret_cast<int32_t*>(lrun_smem) + tid;                        /* [R][T] */
-  unsigned long long* const keycol = reinterpret_cast<unsigned long long*>(lrun_smem) + tid; /* [LIST_LOCAL][T] */
+  unsigned long long* const keycol = reinterpret_cast<unsigned long long*>(lrun_smem) + tid; /* the rebuild's and the long sort's */
   Ctl* const ctl = d.ctl;
   const int n = d.n, K = L.K;
   /* Consecutive slots to consecutive threads; with long lists warp by warp

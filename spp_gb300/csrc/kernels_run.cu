@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(run_threads(PER_SM), PER_SM) k_run(const __gri
   const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
   const int R = run_rows(d.cap, LANES, PER_SM);
   int32_t* const rows = reinterpret_cast<int32_t*>(run_smem) + tid;                        /* [R][T] */
-  unsigned long long* const keycol = reinterpret_cast<unsigned long long*>(run_smem) + tid; /* [LIST_LOCAL][T] */
+  unsigned long long* const keycol = reinterpret_cast<unsigned long long*>(run_smem) + tid; /* the rebuild's and the long sort's */
   int32_t* const ring = reinterpret_cast<int32_t*>(run_smem + (size_t)R * 4 * T) + tid;     /* [4][T] */
   Cold<PER_SM> cold(reinterpret_cast<float*>(run_smem + (size_t)(R * 4 + (BEADLIKE ? RING_SMEM : 0)) * T) + tid, T);
   Ctl* const ctl = d.ctl;

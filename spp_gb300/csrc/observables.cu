@@ -412,7 +412,7 @@ int grid_build(SppSystem* s, double range, size_t nbins, size_t nedges, Grid* g,
   launch_scan_u32(g->count, (uint32_t)nc, g->tmp, g->start, *st, nullptr);
   k_obs_scatter<<<nblk(g->n), SPP_BLOCK, 0, *st>>>(*g);
   OCUDA(cudaGetLastError());
-  spp_internal_count_launches(s, 5);
+  spp_internal_count_launches(s, 4);
   return SPP_OK;
 }
 

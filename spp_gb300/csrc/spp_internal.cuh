@@ -128,10 +128,10 @@ void spp_internal_set_error(const char* msg);
 /* kernels_cells.cu */
 void launch_bin_count(const SppConsts& k, const DevState& d, cudaStream_t s, int64_t* launches);
 void launch_scan(const DevState& d, cudaStream_t s, int64_t* launches);
-/* exclusive scan of n <= scan_max_elements() counts; block_tmp holds
- * ceil(n / 4096) entries */
-void launch_scan_u32(const uint32_t* in, uint32_t n, uint32_t* block_tmp, uint32_t* out,
-                     cudaStream_t s, int64_t* launches);
+/* exclusive scan of n counts; block_tmp holds ceil(n / 4096) entries; counts
+ * and out start on 16-byte boundaries */
+void launch_scan_u32(uint32_t* counts, uint32_t n, uint32_t* block_tmp, uint32_t* out, cudaStream_t s,
+                     int64_t* launches);
 /* the same for a step's cell counts: out has one entry more (the total), and
  * the counts are cleared as they are read */
 void launch_scan_counts(uint32_t* counts, uint32_t n, uint32_t* block_tmp, uint32_t* out, cudaStream_t s);

@@ -45,26 +45,82 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
   return incl - v + warp_sums[warp];
 }
 
-/* Accepted neighbours are collected as (id << 32 | slot) keys in a per-thread
- * array, insertion-sorted there (lists hold ~5 entries at unit density) and
- * written once; lists longer than the array fall back to sorting in place.
- * LIST_LOCAL keys are kept in shared memory per thread (a column of a
- * [LIST_LOCAL][threads] array: conflict-free); entries up to LIST_TAIL are
- * inserted in order in global memory, a list longer than that is finished
- * by sort_queued_list. */
-#ifndef SPP_LIST_LOCAL
-#define SPP_LIST_LOCAL 12
-#endif
-constexpr int LIST_LOCAL = SPP_LIST_LOCAL;
-#ifndef SPP_LIST_TAIL
-#define SPP_LIST_TAIL 16
-#endif
-constexpr int LIST_TAIL = SPP_LIST_TAIL;
+/* Accepted neighbours are collected in visiting order, the slots of the first
+ * LIST_LOCAL in the calling thread's column of shared memory (conflict-free),
+ * the rest in the list itself.  A list that fits the column is put in order by
+ * a sorting network in registers over (order word << 4 | place in the column)
+ * and written once; a longer one is queued for sort_queued_list. */
+constexpr int LIST_LOCAL = 16;
+constexpr int LIST_TRIP = 2;   /* candidates in flight */
 
 /* spp_list_order with the lane count known at compile time */
 template <int LANES>
 __device__ __forceinline__ uint32_t list_order(uint32_t id) {
   return LANES == 1 ? id : ((id & 3u) << 30) | (id >> 2);
+}
+
+/* Batcher's odd-even merge sort (K. E. Batcher, Sorting networks and their
+ * applications, 1968) of key[LO .. LO + N - 1]; entries from LIVE on hold the
+ * largest key throughout, so comparisons with them are left out. */
+template <int LIVE>
+struct SortNetwork {
+  template <int A, int B>
+  static __device__ __forceinline__ void order(uint32_t* key) {
+    if constexpr (B < LIVE) {
+      const uint32_t lo = min(key[A], key[B]), hi = max(key[A], key[B]);
+      key[A] = lo;
+      key[B] = hi;
+    }
+  }
+  template <int A, int END, int R, int STEP>
+  static __device__ __forceinline__ void pairs(uint32_t* key) {
+    if constexpr (A + R < END) {
+      order<A, A + R>(key);
+      pairs<A + STEP, END, R, STEP>(key);
+    }
+  }
+  template <int LO, int N, int R>
+  static __device__ __forceinline__ void merge(uint32_t* key) {
+    if constexpr (2 * R < N) {
+      merge<LO, N, 2 * R>(key);
+      merge<LO + R, N, 2 * R>(key);
+      pairs<LO + R, LO + N, R, 2 * R>(key);
+    } else {
+      order<LO, LO + R>(key);
+    }
+  }
+  template <int LO, int N>
+  static __device__ __forceinline__ void sort(uint32_t* key) {
+    if constexpr (N > 1 && LO < LIVE) {
+      sort<LO, N / 2>(key);
+      sort<LO + N / 2, N / 2>(key);
+      merge<LO, N, 1>(key);
+    }
+  }
+};
+
+/* The cnt <= LIVE collected slots of a thread (col[q * stride]) into its list
+ * in order; returns the neighbours per id % 4 for LANES > 1. */
+template <int LANES, int LIVE>
+__device__ __forceinline__ unsigned long long write_sorted_list(const DevState& d, int i, uint32_t cnt,
+                                                                const uint32_t* col, int stride) {
+  unsigned long long lane_cnt = 0;
+  uint32_t key[LIVE <= 8 ? 8 : 16];
+#pragma unroll
+  for (int q = 0; q < (LIVE <= 8 ? 8 : 16); ++q) {
+    key[q] = 0xffffffffu;
+    if (q < LIVE && (uint32_t)q < cnt) {
+      const uint32_t id = d.id_alt[col[q * stride]];
+      if (LANES > 1) lane_cnt += 1ull << (16 * (id & 3u));
+      /* ids below 2^28, so the order word fits 28 bits */
+      key[q] = (LANES == 1 ? id : ((id & 3u) << 26) | (id >> 2)) << 4 | (uint32_t)q;
+    }
+  }
+  SortNetwork<LIVE>::template sort<0, (LIVE <= 8 ? 8 : 16)>(key);
+#pragma unroll
+  for (int q = 0; q < LIVE; ++q)
+    if ((uint32_t)q < cnt) d.nbr[(size_t)q * d.n + i] = (int32_t)col[(key[q] & 15u) * stride];
+  return lane_cnt;
 }
 
 /* The list of the particle in slot i (position p) from the cell-ordered
@@ -75,69 +131,30 @@ __device__ __forceinline__ uint32_t list_order(uint32_t id) {
  * The 3 x 3 cells are visited row by row with the three cells' ranges of a
  * row loaded together (three dependent round trips per particle instead of
  * nine) and walked as one sequence, two candidates per trip with both
- * candidates' positions and ids in flight; Morton keys built from per-axis
+ * candidates' positions in flight; Morton keys built from per-axis
  * spreads, candidates read as (x, y) only, and the minimum image skipped for
  * particles far from the box edges (where it changes no separation within
  * the list radius, and a candidate across the edge is rejected either way).
  * Measured at the 1M workload 600 steps in (whole rebuild, us): 151.7 with
  * a cell-by-cell walk, 148.4 with rows one candidate per trip, 139.6 with
- * rows two per trip (40 registers; 141.9 when held to 32), 136.8 with the
- * ids loaded with the positions. */
+ * rows two per trip (40 registers; 141.9 when held to 32).  The order comes
+ * at the end, all lanes in step, instead of by insertion as candidates are
+ * accepted: 134 -> 105 200 steps in; resident runs of 16,384 particles 62.5
+ * -> 56.6 us a step (one candidate per trip 58.5), 163,840 beads 24.7 ->
+ * 22.1. */
 template <int LANES>
 __device__ __forceinline__ uint32_t build_particle_list(const SppConsts& k, const DevState& d, int i, float4 p,
-                                                        unsigned long long* col, int stride) {
+                                                        uint32_t* col, int stride) {
   uint32_t cnt = 0;
-  unsigned long long lane_cnt = 0;   /* neighbours per id % 4, 16 bits each */
-#define keys(q) col[(q) * stride]
   int cx, cy;
   cell_key(k, d, p.x, p.y, &cx, &cy);
   const int D = d.D;
   const uint32_t cap = (uint32_t)d.cap;
-  /* one candidate j (cell-ordered slot) */
-  auto visit = [&](uint32_t j, uint32_t idj, float dx, float dy, float d2) {
-    if (d2 < k.rlist2) {
-      const unsigned long long key =
-          ((unsigned long long)list_order<LANES>(idj) << 32) | (unsigned long long)j;
-      if (LANES > 1) lane_cnt += 1ull << (16 * (idj & 3u));
-      if (cnt < (uint32_t)LIST_LOCAL) {
-        /* the order words are unique, so comparing them orders the keys */
-        const uint32_t ko = (uint32_t)(key >> 32);
-        int pos = (int)cnt;
-        while (pos > 0 && (uint32_t)(keys(pos - 1) >> 32) > ko) {
-          keys(pos) = keys(pos - 1);
-          --pos;
-        }
-        keys(pos) = key;
-      } else if (cnt < cap && cnt < (uint32_t)LIST_TAIL) {
-        /* a longer list: the first LIST_LOCAL keys are still local;
-         * keep the next ones sorted in place in global memory */
-        int pos = (int)cnt;
-        while (pos > LIST_LOCAL) {
-          const int32_t prev = d.nbr[(size_t)(pos - 1) * d.n + i];
-          if (list_order<LANES>(d.id_alt[prev]) < (uint32_t)(key >> 32)) break;
-          d.nbr[(size_t)pos * d.n + i] = prev;
-          --pos;
-        }
-        if (pos == LIST_LOCAL && keys(LIST_LOCAL - 1) > key) {
-          /* belongs among the local keys: swap with the local maximum */
-          unsigned long long moved = keys(LIST_LOCAL - 1);
-          int lp = LIST_LOCAL - 1;
-          while (lp > 0 && keys(lp - 1) > key) {
-            keys(lp) = keys(lp - 1);
-            --lp;
-          }
-          keys(lp) = key;
-          d.nbr[(size_t)pos * d.n + i] = (int32_t)(uint32_t)moved;
-        } else {
-          d.nbr[(size_t)pos * d.n + i] = (int32_t)j;
-        }
-      } else if (cnt < cap) {
-        /* a long list: the rest is appended unsorted and k_sort_long
-         * orders the whole list */
-        d.nbr[(size_t)cnt * d.n + i] = (int32_t)j;
-      }
-      ++cnt;
-    }
+  /* an accepted candidate (cell-ordered slot) */
+  auto take = [&](uint32_t j) {
+    if (cnt < (uint32_t)LIST_LOCAL) col[cnt * stride] = j;
+    else if (cnt < cap) d.nbr[(size_t)cnt * d.n + i] = (int32_t)j;
+    ++cnt;
   };
   const int wrap = !(k.closed || (fabsf(p.x) < k.interior && fabsf(p.y) < k.interior));
   uint32_t mx[3];
@@ -168,32 +185,43 @@ __device__ __forceinline__ uint32_t build_particle_list(const SppConsts& k, cons
     auto slot_of = [&](uint32_t t) {
       return t < c[0] ? s0[0] + t : (t < c01 ? s0[1] + (t - c[0]) : s0[2] + (t - c01));
     };
-    for (uint32_t t = 0; t < total; t += 2) {
-      const uint32_t ja = slot_of(t);
-      const uint32_t jb = t + 1 < total ? slot_of(t + 1) : ja;
-      const float2 qa = reinterpret_cast<const float2*>(d.pos_alt)[2 * (size_t)ja];
-      const float2 qb = reinterpret_cast<const float2*>(d.pos_alt)[2 * (size_t)jb];
-      /* both ids with the positions: an accepted candidate's key does not
-       * wait on a second load */
-      const uint32_t ida = d.id_alt[ja], idb = d.id_alt[jb];
-      float dxa, dya, dxb, dyb;
-      const float d2a = wrap ? spp_pair_sep(&k, 1, p.x, p.y, qa.x, qa.y, &dxa, &dya)
-                             : spp_pair_sep(&k, 0, p.x, p.y, qa.x, qa.y, &dxa, &dya);
-      const float d2b = wrap ? spp_pair_sep(&k, 1, p.x, p.y, qb.x, qb.y, &dxb, &dyb)
-                             : spp_pair_sep(&k, 0, p.x, p.y, qb.x, qb.y, &dxb, &dyb);
-      if ((int)ja != i) visit(ja, ida, dxa, dya, d2a);
-      if (t + 1 < total && (int)jb != i) visit(jb, idb, dxb, dyb, d2b);
+    for (uint32_t t = 0; t < total; t += LIST_TRIP) {
+      uint32_t j[LIST_TRIP];
+      float2 q[LIST_TRIP];
+#pragma unroll
+      for (int u = 0; u < LIST_TRIP; ++u) {
+        j[u] = t + u < total ? slot_of(t + u) : (uint32_t)i;
+        q[u] = reinterpret_cast<const float2*>(d.pos_alt)[2 * (size_t)j[u]];
+      }
+      float d2[LIST_TRIP];
+#pragma unroll
+      for (int u = 0; u < LIST_TRIP; ++u) {
+        float dx, dy;
+        d2[u] = wrap ? spp_pair_sep(&k, 1, p.x, p.y, q[u].x, q[u].y, &dx, &dy)
+                     : spp_pair_sep(&k, 0, p.x, p.y, q[u].x, q[u].y, &dx, &dy);
+      }
+#pragma unroll
+      for (int u = 0; u < LIST_TRIP; ++u)
+        if (d2[u] < k.rlist2 && (int)j[u] != i) take(j[u]);
     }
   }
-  const uint32_t nloc = cnt < (uint32_t)LIST_LOCAL ? cnt : (uint32_t)LIST_LOCAL;
-  const uint32_t nw = nloc < cap ? nloc : cap;
-  for (uint32_t q = 0; q < nw; ++q) d.nbr[(size_t)q * d.n + i] = (int32_t)(uint32_t)keys(q);
+  unsigned long long lane_cnt = 0;   /* neighbours per id % 4, 16 bits each */
+  const bool queued = cnt > (uint32_t)LIST_LOCAL || d.n > 1 << 28;
+  const uint32_t in_order = queued || cnt > cap ? 0u : cnt;
+  const uint32_t longest = __reduce_max_sync(__activemask(), in_order);
+  if (longest > 12u) lane_cnt = write_sorted_list<LANES, 16>(d, i, in_order, col, stride);
+  else if (longest > 8u) lane_cnt = write_sorted_list<LANES, 12>(d, i, in_order, col, stride);
+  else lane_cnt = write_sorted_list<LANES, 8>(d, i, in_order, col, stride);
+  if (in_order < cnt) {   /* the queue's, or too long for the list (the run stops and grows it) */
+    const uint32_t held = cnt < cap ? cnt : cap;
+    for (uint32_t q = 0; q < held && q < (uint32_t)LIST_LOCAL; ++q) d.nbr[(size_t)q * d.n + i] = (int32_t)col[q * stride];
+    if (LANES > 1)
+      for (uint32_t q = 0; q < held; ++q) lane_cnt += 1ull << (16 * (d.id_alt[d.nbr[(size_t)q * d.n + i]] & 3u));
+    if (queued) d.long_q[atomicAdd(&d.ctl->long_n, 1u)] = i;
+  }
   d.nn[i] = (int32_t)(cnt < cap ? cnt : cap);
   if (LANES > 1) d.nn_lanes[i] = lane_cnt;   /* meaningful when the list fits */
-  if (cnt > (uint32_t)LIST_TAIL && cap > (uint32_t)LIST_TAIL)
-    d.long_q[atomicAdd(&d.ctl->long_n, 1u)] = i;
   d.ref[i] = make_float2(p.x, p.y);
-#undef keys
   return cnt;
 }
 
@@ -296,7 +324,7 @@ __device__ __forceinline__ void insertion_sort_list(const SppConsts& k, const De
   }
 }
 
-/* A queued list (longer than LIST_TAIL) put in order by the calling warp. */
+/* A queued list (longer than LIST_LOCAL) put in order by the calling warp. */
 __device__ __forceinline__ void sort_queued_list(const SppConsts& k, const DevState& d, int i) {
   if (!spp_index_ok(d.ctl, i, d.n)) return;
   const int m = d.nn[i];

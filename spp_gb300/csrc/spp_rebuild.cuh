@@ -7,7 +7,7 @@
 
 namespace {
 
-/* Shared memory per thread: the list build's LIST_LOCAL keys, then the keys
+/* Shared memory per thread: the list build's LIST_LOCAL slots, then the keys
  * of the long-list sort (RUN_SORT_MAX per warp); between rebuilds the same
  * bytes hold the first run_rows() entries of the thread's neighbour segment
  * (later entries are read from global memory): 32 of them, or 64 where the
@@ -15,7 +15,7 @@ namespace {
  * block per SM leaves the room. */
 constexpr int RUN_SORT_MAX = 512;
 constexpr int RUN_SMEM = RUN_SORT_MAX * 8 / 32;
-static_assert(RUN_SMEM >= LIST_LOCAL * 8, "the build's keys");
+static_assert(RUN_SMEM >= LIST_LOCAL * 4, "the build's slots");
 constexpr int RUN_ROWS = RUN_SMEM / 4, RUN_ROWS_LONG = 64;
 __host__ __device__ inline int run_rows(int cap, int lanes, int per_sm) {
   return per_sm == 1 && cap > 3 * lanes * RUN_ROWS / 4 ? RUN_ROWS_LONG : RUN_ROWS;
@@ -24,7 +24,7 @@ __host__ __device__ inline int run_rows(int cap, int lanes, int per_sm) {
  * neighbours in flight. */
 constexpr int RUN_LONG = 12;
 
-/* A queued list (longer than LIST_TAIL) put in order by the calling warp, as
+/* A queued list (longer than LIST_LOCAL) put in order by the calling warp, as
  * sort_queued_list (spp_list.cuh) does, by a bitonic network over keys in
  * the warp's shared memory: loops instead of registers, a tenth of the code. */
 __device__ __forceinline__ void run_sort_list(const SppConsts& k, const DevState& d, int i, unsigned long long* keys) {
@@ -74,7 +74,7 @@ template <int LANES>
 __device__ __noinline__ int run_rebuild(const SppConsts& k, const DevState& d, int i, bool head, float4 p,
                                         float th0, uint32_t pid, unsigned long long* keycol, unsigned* target,
                                         unsigned* s_word) {
-  const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, n = d.n;
+  const int T = blockDim.x, tid = threadIdx.x, n = d.n;
   const int gthreads = gridDim.x * T, gtid = blockIdx.x * T + tid;
   Ctl* const ctl = d.ctl;
   /* arrive and wait in one; false when the block must leave */
@@ -90,19 +90,11 @@ __device__ __noinline__ int run_rebuild(const SppConsts& k, const DevState& d, i
   };
   uint32_t key = 0u, rank = 0u;
   if (gtid == 0) ctl->long_n = 0u;
-  {
-    const unsigned heads = __ballot_sync(0xffffffffu, head);
-    if (head) {
-      int cx, cy;
-      key = cell_key(k, d, p.x, p.y, &cx, &cy);
-      if (!spp_index_ok(ctl, key, d.n_keys)) key = 0u;
-      const unsigned peers = __match_any_sync(heads, key);
-      const int leader = __ffs(peers) - 1;
-      uint32_t base = 0u;
-      if (lane == leader) base = atomicAdd(&d.cell_count[key], (uint32_t)__popc(peers));
-      base = __shfl_sync(peers, base, leader);
-      rank = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-    }
+  if (head) {
+    int cx, cy;
+    key = cell_key(k, d, p.x, p.y, &cx, &cy);
+    if (!spp_index_ok(ctl, key, d.n_keys)) key = 0u;
+    rank = atomicAdd(&d.cell_count[key], 1u);
   }
   if (!barrier()) return RUN_LOST;
   if (!grid_scan(d.cell_count, d.cell_start, d.n_keys, d.run_sums, barrier)) return RUN_LOST;
@@ -123,7 +115,7 @@ __device__ __noinline__ int run_rebuild(const SppConsts& k, const DevState& d, i
     uint32_t cnt = 0u;
     if (tid < T / LANES && ib < n) {
       const float4 q = d.pos_alt[ib];
-      cnt = build_particle_list<LANES>(k, d, ib, q, keycol, T);
+      cnt = build_particle_list<LANES>(k, d, ib, q, reinterpret_cast<uint32_t*>(keycol - tid) + tid, T);
       adopt_sorted_particle(d, ib, q);
     }
     note_list_lengths(d, cnt);

@@ -49,3 +49,18 @@ def test_body_frame(gpu_lib, n, L, lattice, lx, ly, gx, gy):
         s.upload(x, y, th)
         got = s.pair_distribution(lx, ly, gx, gy)
     assert np.array_equal(got, O.pair_distribution32(x, y, c, sn, lx, ly, gx, gy))
+
+
+def test_radial_on_a_grid_of_many_cells(gpu_lib):
+    """17.6 million cells: more tiles of the scan than one block scans."""
+    L, n = 420.0, 3000
+    g = np.random.default_rng(5)
+    c = (g.random((n // 3, 2)) * 2 * L - L)
+    xy = (np.concatenate([c, c + 0.05 + 0.1 * g.random(c.shape), c - 0.1 * g.random(c.shape)])).astype(np.float32)
+    xy = np.clip(xy, -L, np.nextafter(np.float32(L), np.float32(0.0)))
+    x, y = np.ascontiguousarray(xy[:, 0]), np.ascontiguousarray(xy[:, 1])
+    want = O.radial32(x, y, L, 0.2, 7)
+    assert want.sum() > n / 2
+    with System(configs.vicsek_config(n=n, L=L)) as s:
+        s.upload(x, y, np.zeros(n, np.float32))
+        assert np.array_equal(s.radial_distribution(0.2, 7), want)
