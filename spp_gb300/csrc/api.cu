@@ -326,7 +326,7 @@ int enqueue_rebuild(SppSystem* s, cudaStream_t st, int64_t* launches) {
   CUDA_TRY(cudaMemsetAsync(s->d.cell_count, 0, sizeof(uint32_t) * s->d.n_keys, st));
   launch_bin_count(s->k, s->d, st, launches);
   launch_scan(s->d, st, launches);
-  launch_scatter(s->d, st, launches);
+  launch_scatter(s->d, false, st, launches);
   launch_build_list(s->k, s->d, s->uses_list ? 1 : 0, st, launches);
   CUDA_TRY(cudaGetLastError());
   return SPP_OK;
@@ -344,7 +344,7 @@ int enqueue_step(SppSystem* s, cudaStream_t st, bool capture, int64_t* launches)
     CUDA_TRY(cudaMemsetAsync(s->d.cell_count, 0, sizeof(uint32_t) * s->d.n_keys, st));
     launch_bin_count(s->k, s->d, st, launches);
     launch_scan(s->d, st, launches);
-    launch_scatter(s->d, st, launches);
+    launch_scatter(s->d, true, st, launches);
     launch_vicsek_step(s->k, s->d, st, launches);
     CUDA_TRY(cudaGetLastError());
     return SPP_OK;

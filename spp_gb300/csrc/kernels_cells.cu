@@ -23,6 +23,7 @@
  */
 #include "spp_internal.cuh"
 #include "spp_list.cuh"
+#include "spp_pack.cuh"
 
 namespace {
 
@@ -138,6 +139,8 @@ __global__ void __launch_bounds__(SCAN_COUNT_THREADS) k_scan_counts(uint32_t* co
   }
 }
 
+/* VICSEK: the copy holds a heading's packed parts in place of (cos, sin). */
+template <bool VICSEK>
 __global__ void __launch_bounds__(SPP_BLOCK) k_scatter(DevState d) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.n) return;
@@ -145,7 +148,12 @@ __global__ void __launch_bounds__(SPP_BLOCK) k_scatter(DevState d) {
   if (!spp_index_ok(d.ctl, key, d.n_keys)) return;
   uint32_t dst = d.cell_start[key] + d.rank[i];
   if (!spp_index_ok(d.ctl, dst, d.n)) return;
-  d.pos_alt[dst] = d.pos[i];
+  float4 p = d.pos[i];
+  if (VICSEK) {
+    p.z = pack_parts(fx_parts(p.z));
+    p.w = pack_parts(fx_parts(p.w));
+  }
+  d.pos_alt[dst] = p;
   d.theta_alt[dst] = d.theta[i];
   d.img_alt[dst] = d.img[i];
   d.id_alt[dst] = d.id[i];
@@ -295,9 +303,10 @@ void launch_scan(const DevState& d, cudaStream_t s, int64_t* launches) {
   launch_scan_u32(d.cell_count, d.n_keys, d.scan_tmp, d.cell_start, s, launches);
 }
 
-void launch_scatter(const DevState& d, cudaStream_t s, int64_t* launches) {
+void launch_scatter(const DevState& d, bool vicsek, cudaStream_t s, int64_t* launches) {
   if (d.n == 0) return;
-  k_scatter<<<blocks_for(d.n), SPP_BLOCK, 0, s>>>(d);
+  if (vicsek) k_scatter<true><<<blocks_for(d.n), SPP_BLOCK, 0, s>>>(d);
+  else k_scatter<false><<<blocks_for(d.n), SPP_BLOCK, 0, s>>>(d);
   if (launches) *launches += 1;
 }
 

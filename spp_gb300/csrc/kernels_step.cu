@@ -24,6 +24,7 @@
  * rebuilt every step at dt = 1).
  */
 #include "spp_internal.cuh"
+#include "spp_pack.cuh"
 #include <mutex>
 
 namespace {
@@ -619,45 +620,113 @@ __global__ void __launch_bounds__(SPP_STAGE_BLOCK, KIND == SPP_KIND_CHAIN ? 1024
 #endif
 }
 
+/* The candidates of a particle at p (cell (cx, cy), slot i): the 3 x 3 cells,
+ * a row's three ranges walked as one sequence, VICSEK_TRIP candidates in
+ * flight.  WRAP: some image may be nearer.
+ * Bound by the walk's loads and instructions.  Whole steps (us; N = 200,003 /
+ * 499,979 at density 2, eta = 0.3, 200 steps in): cell by cell, one candidate
+ * at a time, headings split into their parts for every candidate, 68.5 /
+ * 122.5 vector sum, 57.1 / 96.2 angles, 226 / 343 with push; now 35.4 / 60.1,
+ * 42.5 / 68.4 and 144 / 211.  Two candidates in flight: 42.9 / 70.5, 44.0 /
+ * 70.8, 166 / 242; four: 37.9 / 63.9, 45.1 / 71.9, 145 / 212. */
+constexpr int VICSEK_TRIP = 3;
+template <int MODEL, bool WRAP>
+__device__ __forceinline__ void vicsek_walk(const SppConsts& k, const DevState& d, int i, float4 p, int cx, int cy,
+                                            SppAcc* a, PackedSum* sx, PackedSum* sy) {
+  const int D = d.D;
+  uint32_t mx[3];
+#pragma unroll
+  for (int o = 0; o < 3; ++o) {
+    int nx = cx + o - 1;
+    nx = nx < 0 ? nx + D : (nx >= D ? nx - D : nx);
+    mx[o] = spp_morton_spread((uint32_t)nx);
+  }
+#pragma unroll 1
+  for (int oy = -1; oy <= 1; ++oy) {
+    int ny = cy + oy;
+    ny = ny < 0 ? ny + D : (ny >= D ? ny - D : ny);
+    const uint32_t my = spp_morton_spread((uint32_t)ny) << 1;
+    uint32_t s0[3], c[3];
+#pragma unroll
+    for (int o = 0; o < 3; ++o) {
+      const uint32_t kk = mx[o] | my;
+      s0[o] = c[o] = 0u;
+      if (!spp_index_ok(d.ctl, kk, d.n_keys)) continue;
+      s0[o] = d.cell_start[kk];
+      c[o] = d.cell_count[kk];
+      if (!spp_index_ok(d.ctl, (long long)s0[o] + c[o], (long long)d.n + 1)) c[o] = 0u;
+    }
+    const uint32_t c01 = c[0] + c[1], total = c01 + c[2];
+    const uint32_t m1 = s0[1] - c[0], m2 = s0[2] - c01;   /* slot = t + m (wraps as unsigned) */
+    for (uint32_t t = 0; t < total; t += VICSEK_TRIP) {
+      uint32_t j[VICSEK_TRIP];
+      float4 q[VICSEK_TRIP];
+#pragma unroll
+      for (int u = 0; u < VICSEK_TRIP; ++u) {
+        const uint32_t v = t + u;
+        j[u] = v + (v < c[0] ? s0[0] : (v < c01 ? m1 : m2));
+        if (v < total) q[u] = __ldg(d.pos_alt + j[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < VICSEK_TRIP; ++u) {
+        if (t + u >= total) continue;
+        float dx, dy;
+        const float d2 = spp_pair_sep(&k, WRAP, p.x, p.y, q[u].x, q[u].y, &dx, &dy);
+        if (!(d2 < k.ral2)) continue;
+        if (MODEL != SPP_MODEL_VICSEK && (int)j[u] == i) continue;   /* the vector sum counts the particle itself */
+        a->cnt += 1;
+        if (MODEL == SPP_MODEL_VICSEK_REF_ANGLE) {
+          spp_fx_add_guarded(&a->at, d.theta_alt[j[u]], &a->ovf);
+          continue;
+        }
+        packed_add(sx, q[u].z);
+        packed_add(sy, q[u].w);
+        if (MODEL == SPP_MODEL_VICSEK_REF_VECTOR && d2 < k.rpush2 && d2 > 0.0f) spp_push_vicsek(&k, a, dx, dy, d2);
+      }
+    }
+  }
+}
+
+/* From the cell-ordered copy (headings packed, k_scatter<true>) back into the
+ * primary arrays. */
+template <int MODEL>
 __global__ void __launch_bounds__(SPP_BLOCK) k_vicsek_step(SppConsts k, DevState d) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < d.n) {
-    const uint32_t step = d.ctl->step;
     const float4 p = d.pos_alt[i];
-    const float th0 = d.theta_alt[i];
-    const uint32_t id = d.id_alt[i];
-    const int cx = spp_cell_coord(p.x, k.L, k.L2, d.D, SPP_BIN_GEOMETRIC);
-    const int cy = spp_cell_coord(p.y, k.L, k.L2, d.D, SPP_BIN_GEOMETRIC);
     const int D = d.D;
-    const int need_theta = (k.model == SPP_MODEL_VICSEK_REF_ANGLE);
+    const int cx = spp_cell_coord(p.x, k.L, k.L2, D, SPP_BIN_GEOMETRIC);
+    const int cy = spp_cell_coord(p.y, k.L, k.L2, D, SPP_BIN_GEOMETRIC);
     SppAcc a;
     spp_acc_zero(&a);
-    for (int oy = -1; oy <= 1; ++oy) {
-      int ny = cy + oy;
-      ny = ny < 0 ? ny + D : (ny >= D ? ny - D : ny);
-      for (int ox = -1; ox <= 1; ++ox) {
-        int nx = cx + ox;
-        nx = nx < 0 ? nx + D : (nx >= D ? nx - D : nx);
-        const uint32_t kk = spp_morton((uint32_t)nx, (uint32_t)ny);
-        if (!spp_index_ok(d.ctl, kk, d.n_keys)) continue;
-        const uint32_t s0 = d.cell_start[kk], c = d.cell_count[kk];
-        if (!spp_index_ok(d.ctl, (long long)s0 + c, (long long)d.n + 1)) continue;
-        for (uint32_t j = s0; j < s0 + c; ++j) {
-          const float4 q = __ldg(d.pos_alt + j);
-          const float thj = need_theta ? d.theta_alt[j] : 0.0f;
-          spp_pair_vicsek(&k, &a, p.x, p.y, q.x, q.y, q.z, q.w, thj, (int)j == i);
-        }
-      }
+    PackedSum sx = {0, 0}, sy = {0, 0};
+    /* a candidate of an interior cell is nearest as it is (or two cells away,
+     * beyond every cutoff), and a closed box has no images */
+    const int plain = k.closed || (cx >= 1 && cx <= D - 2 && cy >= 1 && cy <= D - 2);
+    if (__all_sync(__activemask(), plain)) vicsek_walk<MODEL, false>(k, d, i, p, cx, cy, &a, &sx, &sy);
+    else vicsek_walk<MODEL, true>(k, d, i, p, cx, cy, &a, &sx, &sy);
+    if (MODEL != SPP_MODEL_VICSEK_REF_ANGLE) {
+      const spp_fx fx = packed_value(sx, a.cnt), fy = packed_value(sy, a.cnt);
+      a.ax.hi += fx.hi;
+      a.ax.lo += fx.lo;
+      a.ay.hi += fy.hi;
+      a.ay.lo += fy.lo;
     }
-    if (k.closed && k.model == SPP_MODEL_VICSEK_REF_ANGLE) spp_vicsek_walls(&k, &a, p.x, p.y, th0);
+    float th0 = 0.0f, c0 = 0.0f, s0 = 0.0f;
+    if (MODEL != SPP_MODEL_VICSEK) {
+      th0 = d.theta_alt[i];
+      spp_sincosf(th0, &s0, &c0);   /* as the step before left them */
+    }
+    if (MODEL == SPP_MODEL_VICSEK_REF_ANGLE && k.closed) spp_vicsek_walls(&k, &a, p.x, p.y, th0);
     if (a.ovf) atomicOr(&d.ctl->fx_overflow, 1u);
-    const spp_u32x4 r = spp_draw_k(&k, id, step, SPP_RNG_VICSEK);
+    const uint32_t id = d.id_alt[i];
+    const spp_u32x4 r = spp_draw_k(&k, id, d.ctl->step, SPP_RNG_VICSEK);
     float x, y, t, c, s;
     int gx = 0, gy = 0;
-    spp_vicsek_update(&k, &a, p.x, p.y, th0, p.z, p.w, r.v[0], &x, &y, &t, &c, &s, &gx, &gy);
+    spp_vicsek_update(&k, &a, p.x, p.y, th0, c0, s0, r.v[0], &x, &y, &t, &c, &s, &gx, &gy);
     d.pos[i] = make_float4(x, y, c, s);
     d.theta[i] = t;
-    int2 g = d.img_alt[i];
+    const int2 g = d.img_alt[i];
     d.img[i] = make_int2(g.x + gx, g.y + gy);
     d.id[i] = id;
   }
@@ -779,7 +848,11 @@ void prepare_abp_stage() {
 void launch_vicsek_step(const SppConsts& k, const DevState& d, cudaStream_t s, int64_t* launches) {
   int nb = blocks_for(d.n);
   if (nb == 0) nb = 1;
-  k_vicsek_step<<<nb, SPP_BLOCK, 0, s>>>(k, d);
+  switch (k.model) {
+    case SPP_MODEL_VICSEK: k_vicsek_step<SPP_MODEL_VICSEK><<<nb, SPP_BLOCK, 0, s>>>(k, d); break;
+    case SPP_MODEL_VICSEK_REF_ANGLE: k_vicsek_step<SPP_MODEL_VICSEK_REF_ANGLE><<<nb, SPP_BLOCK, 0, s>>>(k, d); break;
+    default: k_vicsek_step<SPP_MODEL_VICSEK_REF_VECTOR><<<nb, SPP_BLOCK, 0, s>>>(k, d); break;
+  }
   if (launches) *launches += 1;
 }
 

@@ -136,7 +136,7 @@ void launch_scan_u32(uint32_t* counts, uint32_t n, uint32_t* block_tmp, uint32_t
  * the counts are cleared as they are read */
 void launch_scan_counts(uint32_t* counts, uint32_t n, uint32_t* block_tmp, uint32_t* out, cudaStream_t s);
 uint32_t scan_max_elements();
-void launch_scatter(const DevState& d, cudaStream_t s, int64_t* launches);
+void launch_scatter(const DevState& d, bool vicsek, cudaStream_t s, int64_t* launches);
 void launch_build_list(const SppConsts& k, const DevState& d, int with_list, cudaStream_t s,
                        int64_t* launches);
 void launch_pairs_count(const SppConsts& k, const DevState& d, float r2, unsigned long long* counter,
