@@ -22,19 +22,25 @@
  *
  * Why: a step of six dependent kernels is bound by their latency.  Measured
  * (one GB300, vector rule, unit density, eta = 0.3, flocking; us per step):
- * N = 4,096 30.9 -> 7.0 (12.8 in one cluster of 16 CTAs, the former path of
- * systems up to 16,384); 16,384 35.4 -> 8.6; 50,001 42.5 -> 17.0; 175,104
- * 59.0 -> 32.6.  What bounds it now: small systems the chain barrier (1.1 us)
+ * N = 4,096 30.9 -> 6.5 (12.8 in one cluster of 16 CTAs, the former path of
+ * systems up to 16,384); 16,384 35.4 -> 8.0; 50,001 42.5 -> 13.6; 175,104
+ * 59.0 -> 27.8.  What bounds it now: small systems the chain barrier (1.1 us)
  * -> counts and first candidates -> the rest of the candidates -> update ->
  * place in the cell (an atomic's round trip) -> stores visible; large ones
- * the candidate walk, whose length is the warp's longest.  Candidates in
- * flight: 2 / 4 / 6 take 8.2 / 7.0 / 6.9 us at N = 4,096 and 22.8 / 19.6 /
- * 18.8 at 50,001 (vector rule), 6 is slower from 87,552 on and for the angle
- * rule.  Without the sorts N = 50,001 takes 28.4, with one every 8 steps as
- * long as with one every 16.
+ * the candidate walk, whose length is the warp's longest.  A second copy of
+ * the walk without images, for warps away from the box edges, and packed
+ * headings that take two additions a term: 7.5 -> 6.9 us at N = 4,096, 25.0 ->
+ * 21.9 at 50,001 and density 2, 52.5 -> 44.3 at 175,000 (with push 197 -> 146).
+ * Candidates in flight, vector rule: 3 / 4 / 6 take 7.3 / 6.9 / 6.6, 24.1 /
+ * 21.9 / 20.0 and 49.6 / 44.3 / 39.8; the other rules, whose terms need the
+ * registers: angles at 50,001 15.9 / 15.7 / 16.7, push 59 / 56 / 55.
+ * Without the sorts N = 50,001 took 28.4 (17.0 with them at the time), with
+ * one every 8 steps as long as with one every 16.
  */
 #include "spp_internal.cuh"
 #include "spp_grid.cuh"
+#include "spp_pack.cuh"
+#include <type_traits>
 
 namespace {
 
@@ -42,41 +48,31 @@ __host__ __device__ constexpr int vrun_threads(int per_sm) { return per_sm == 1 
 
 constexpr uint32_t VRUN_SORT = 16;   /* steps between two sorts of the owners */
 
-/* A bucket entry: position, and the fixed-point parts of cos and sin
- * (spp_fx_add: |hi| <= 32, |lo| <= 2^21) packed as hi << 24 | lo in 24 bits. */
-__device__ __forceinline__ float pack_fx(float v) {
-  spp_fx a = {0, 0};
-  spp_fx_add(&a, v);
-  return __int_as_float((int)((uint32_t)a.hi << 24 | ((uint32_t)a.lo & 0x00ffffffu)));
-}
-__device__ __forceinline__ void add_packed(spp_fx* a, float w) {
-  const int v = __float_as_int(w);
-  a->hi += v >> 24;
-  a->lo += (int)((uint32_t)v << 8) >> 8;
-}
+/* A bucket entry: position, and the packed parts of cos and sin. */
+__device__ __forceinline__ float pack_fx(float v) { return pack_parts(fx_parts(v)); }
+
+/* The sums a particle receives. */
+struct VrunAcc {
+  PackedSum cx, cy;   /* headings of the aligning neighbours */
+  SppAcc a;           /* count, angles (ax, ay: the push terms) */
+};
 
 /* One candidate (entry q, heading thj for the angle rule); the terms of
- * spp_pair_vicsek. */
-template <int MODEL>
-__device__ __forceinline__ void vrun_pair(const SppConsts& k, SppAcc* a, float4 p, float4 q, float thj, bool self) {
+ * spp_pair_vicsek.  WRAP: some image may be nearer. */
+template <int MODEL, bool WRAP>
+__device__ __forceinline__ void vrun_pair(const SppConsts& k, VrunAcc* acc, float4 p, float4 q, float thj, bool self) {
   float dx, dy;
-  const float d2 = spp_sep(&k, p.x, p.y, q.x, q.y, &dx, &dy);
+  const float d2 = spp_pair_sep(&k, WRAP, p.x, p.y, q.x, q.y, &dx, &dy);
   if (!(d2 < k.ral2)) return;
-  if (MODEL == SPP_MODEL_VICSEK) {
-    add_packed(&a->ax, q.z);
-    add_packed(&a->ay, q.w);
-    a->cnt += 1;
-    return;
-  }
-  if (self) return;
-  a->cnt += 1;
+  if (MODEL != SPP_MODEL_VICSEK && self) return;   /* the vector sum counts the particle itself */
+  acc->a.cnt += 1;
   if (MODEL == SPP_MODEL_VICSEK_REF_ANGLE) {
-    spp_fx_add_guarded(&a->at, thj, &a->ovf);
+    spp_fx_add_guarded(&acc->a.at, thj, &acc->a.ovf);
     return;
   }
-  add_packed(&a->ax, q.z);
-  add_packed(&a->ay, q.w);
-  if (d2 < k.rpush2 && d2 > 0.0f) spp_push_vicsek(&k, a, dx, dy, d2);
+  packed_add(&acc->cx, q.z);
+  packed_add(&acc->cy, q.w);
+  if (MODEL == SPP_MODEL_VICSEK_REF_VECTOR && d2 < k.rpush2 && d2 > 0.0f) spp_push_vicsek(&k, &acc->a, dx, dy, d2);
 }
 
 /* Counts are kept for three steps, buckets for two: step t reads count
@@ -90,7 +86,7 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
   constexpr bool ANGLE = MODEL == SPP_MODEL_VICSEK_REF_ANGLE;
   constexpr int NC = (9 + LANES - 1) / LANES;   /* cells per lane */
   constexpr int AT_ONCE = 3;                    /* cells whose loads are issued together */
-  constexpr int DEPTH = 4;                      /* candidates whose loads are issued together */
+    constexpr int DEPTH = MODEL == SPP_MODEL_VICSEK ? 6 : 4;   /* candidates whose loads are issued together */
   __shared__ unsigned s_word;
   __shared__ unsigned long long s_sum[2];
   const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
@@ -198,67 +194,84 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
     }
     const float4* const cand = full ? d.pos_alt : vb.bucket[t & 1];
     const float* const cand_th = full ? d.theta_alt : vb.bucket_th[t & 1];
-    SppAcc a;
-    spp_acc_zero(&a);
+    VrunAcc acc;
+    acc.cx = acc.cy = {0, 0};
+    spp_acc_zero(&acc.a);
     auto cell_of = [&](int c9) -> uint32_t {
       int ny = cy + c9 / 3 - 1, nx = cx + c9 % 3 - 1;
       ny = ny < 0 ? ny + D : (ny >= D ? ny - D : ny);
       nx = nx < 0 ? nx + D : (nx >= D ? nx - D : nx);
       return (uint32_t)ny * (uint32_t)D + (uint32_t)nx;
     };
+    auto walk = [&](auto wrapped) {
+      constexpr bool WRAP = decltype(wrapped)::value;
 #pragma unroll 1
-    for (int m0 = 0; inb && m0 < NC; m0 += AT_ONCE) {
-      /* a cell's candidates: cnt of them from base on; the first of each is
-       * asked for before the count is known (a place not taken holds an
-       * older state, not used) */
-      uint32_t cnt[AT_ONCE], base[AT_ONCE];
-      float4 q[AT_ONCE];
-      float qt[AT_ONCE];
+      for (int m0 = 0; inb && m0 < NC; m0 += AT_ONCE) {
+        /* a cell's candidates: cnt of them from base on; the first of each is
+         * asked for before the count is known (a place not taken holds an
+         * older state, not used) */
+        uint32_t cnt[AT_ONCE], base[AT_ONCE];
+        float4 q[AT_ONCE];
+        float qt[AT_ONCE];
 #pragma unroll
-      for (int m = 0; m < AT_ONCE; ++m) {
-        const int c9 = lane_r + LANES * (m0 + m);
-        const bool is = m0 + m < NC && c9 < 9;
-        const uint32_t cell = cell_of(is ? c9 : 4);
-        cnt[m] = is ? count[cell] : 0u;
-        base[m] = full ? min(d.cell_start[cell], (uint32_t)n - 1u) : cell * (uint32_t)K;
-        q[m] = cand[base[m]];
-        qt[m] = ANGLE ? cand_th[base[m]] : 0.0f;
-      }
-#pragma unroll
-      for (int m = 0; m < AT_ONCE; ++m)
-        if (cnt[m] > 0u)
-          vrun_pair<MODEL>(k, &a, p, q[m], qt[m], lane_r + LANES * (m0 + m) == 4 && rank == 0u);
-      /* the rest of the cells as one sequence, DEPTH at a time: lanes differ
-       * only in its length */
-      int l[AT_ONCE + 1];
-      l[0] = 0;
-#pragma unroll
-      for (int m = 0; m < AT_ONCE; ++m) l[m + 1] = l[m] + max((int)cnt[m] - 1, 0);
-      for (int s = 0; s < l[AT_ONCE]; s += DEPTH) {
-        float4 qs[DEPTH];
-        float ts[DEPTH];
-        bool self[DEPTH];
-#pragma unroll
-        for (int u = 0; u < DEPTH; ++u) {
-          const int v = min(s + u, l[AT_ONCE] - 1);
-          uint32_t at = base[0];
-          int off = -1, c9 = lane_r + LANES * m0;
-#pragma unroll
-          for (int w = 1; w < AT_ONCE; ++w)
-            if (v >= l[w]) {
-              at = base[w];
-              off = l[w] - 1;
-              c9 = lane_r + LANES * (m0 + w);
-            }
-          const uint32_t e = (uint32_t)(v - off);
-          qs[u] = cand[at + e];
-          ts[u] = ANGLE ? cand_th[at + e] : 0.0f;
-          self[u] = c9 == 4 && e == rank;
+        for (int m = 0; m < AT_ONCE; ++m) {
+          const int c9 = lane_r + LANES * (m0 + m);
+          const bool is = m0 + m < NC && c9 < 9;
+          const uint32_t cell = cell_of(is ? c9 : 4);
+          cnt[m] = is ? count[cell] : 0u;
+          base[m] = full ? min(d.cell_start[cell], (uint32_t)n - 1u) : cell * (uint32_t)K;
+          q[m] = cand[base[m]];
+          qt[m] = ANGLE ? cand_th[base[m]] : 0.0f;
         }
 #pragma unroll
-        for (int u = 0; u < DEPTH; ++u)
-          if (s + u < l[AT_ONCE]) vrun_pair<MODEL>(k, &a, p, qs[u], ts[u], self[u]);
+        for (int m = 0; m < AT_ONCE; ++m)
+          if (cnt[m] > 0u)
+            vrun_pair<MODEL, WRAP>(k, &acc, p, q[m], qt[m], lane_r + LANES * (m0 + m) == 4 && rank == 0u);
+        /* the rest of the cells as one sequence, DEPTH at a time: lanes differ
+         * only in its length */
+        int l[AT_ONCE + 1];
+        l[0] = 0;
+#pragma unroll
+        for (int m = 0; m < AT_ONCE; ++m) l[m + 1] = l[m] + max((int)cnt[m] - 1, 0);
+        for (int s = 0; s < l[AT_ONCE]; s += DEPTH) {
+          float4 qs[DEPTH];
+          float ts[DEPTH];
+          bool self[DEPTH];
+#pragma unroll
+          for (int u = 0; u < DEPTH; ++u) {
+            const int v = min(s + u, l[AT_ONCE] - 1);
+            uint32_t at = base[0];
+            int off = -1, c9 = lane_r + LANES * m0;
+#pragma unroll
+            for (int w = 1; w < AT_ONCE; ++w)
+              if (v >= l[w]) {
+                at = base[w];
+                off = l[w] - 1;
+                c9 = lane_r + LANES * (m0 + w);
+              }
+            const uint32_t e = (uint32_t)(v - off);
+            qs[u] = cand[at + e];
+            ts[u] = ANGLE ? cand_th[at + e] : 0.0f;
+            self[u] = c9 == 4 && e == rank;
+          }
+#pragma unroll
+          for (int u = 0; u < DEPTH; ++u)
+            if (s + u < l[AT_ONCE]) vrun_pair<MODEL, WRAP>(k, &acc, p, qs[u], ts[u], self[u]);
+        }
       }
+    };
+    /* a candidate of an interior cell is nearest as it is (or two cells away,
+     * beyond every cutoff), and a closed box has no images */
+    const int plain = !inb || k.closed || (cx >= 1 && cx <= D - 2 && cy >= 1 && cy <= D - 2);
+    if (__all_sync(0xffffffffu, plain)) walk(std::false_type{});
+    else walk(std::true_type{});
+    SppAcc& a = acc.a;
+    if (!ANGLE) {
+      const spp_fx fx = packed_value(acc.cx, a.cnt), fy = packed_value(acc.cy, a.cnt);
+      a.ax.hi += fx.hi;
+      a.ax.lo += fx.lo;
+      a.ay.hi += fy.hi;
+      a.ay.lo += fy.lo;
     }
     if (LANES > 1) {
 #pragma unroll
@@ -381,8 +394,8 @@ bool plan_vrun(const SppConsts& k, const DevState& d, VrunPlan* plan) {
     return false;
   }
   /* As many lanes per particle as there is room for (us per step of the
-   * vector rule, one GB300, lanes 1 / 2 / 4: N = 4,096 13.4 / 9.3 / 7.0; 43,776
-   * 18.1 / 13.6 / 13.2; 87,552 20.5 / 19.7); one block per SM while it holds
+   * vector rule, one GB300, lanes 1 / 2 / 4, before the walk without images: N =
+   * 4,096 13.4 / 9.3 / 7.0; 43,776 18.1 / 13.6 / 13.2; 87,552 20.5 / 19.7); one block per SM while it holds
    * the threads. */
   const int64_t room = (int64_t)2 * sms * vrun_threads(2);
   const int lanes = 4 * (int64_t)d.n <= room ? 4 : (2 * (int64_t)d.n <= room ? 2 : 1);
