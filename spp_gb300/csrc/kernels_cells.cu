@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(SPP_BLOCK) k_scatter(DevState d) {
  * for 5 neighbours).  At N = 1,048,576, ABP, unit density, 200 steps in: 87.6
  * us a launch when accepted neighbours were inserted in id order as they came
  * (each lane its own depth), 61 with them collected and put in order by a
- * network (build_particle_list); a whole rebuild 134 -> 101.  40 registers
+ * network (build_particle_list); a whole rebuild 134 -> 98.  40 registers
  * for six blocks per SM; four or five are not faster.
  * Verlet list from the cell-ordered copy (alt), then the copy moves back
  * into the primary arrays. with_list == 0 only copies (no list).  The copy

@@ -139,9 +139,10 @@ __device__ __forceinline__ unsigned long long write_sorted_list(const DevState& 
  * a cell-by-cell walk, 148.4 with rows one candidate per trip, 139.6 with
  * rows two per trip (40 registers; 141.9 when held to 32).  The order comes
  * at the end, all lanes in step, instead of by insertion as candidates are
- * accepted: 134 -> 105 200 steps in; resident runs of 16,384 particles 62.5
- * -> 56.6 us a step (one candidate per trip 58.5), 163,840 beads 24.7 ->
- * 22.1. */
+ * accepted, and a candidate is stored whether taken or not (98 against 101 with
+ * a branch): 134 -> 98 200 steps in; 50 steps of resident runs of 16,384
+ * particles 1,254 -> 1,120 us (one candidate per trip 1,170), of 163,840 beads
+ * 1,240 -> 1,107. */
 template <int LANES>
 __device__ __forceinline__ uint32_t build_particle_list(const SppConsts& k, const DevState& d, int i, float4 p,
                                                         uint32_t* col, int stride) {
@@ -150,12 +151,6 @@ __device__ __forceinline__ uint32_t build_particle_list(const SppConsts& k, cons
   cell_key(k, d, p.x, p.y, &cx, &cy);
   const int D = d.D;
   const uint32_t cap = (uint32_t)d.cap;
-  /* an accepted candidate (cell-ordered slot) */
-  auto take = [&](uint32_t j) {
-    if (cnt < (uint32_t)LIST_LOCAL) col[cnt * stride] = j;
-    else if (cnt < cap) d.nbr[(size_t)cnt * d.n + i] = (int32_t)j;
-    ++cnt;
-  };
   const int wrap = !(k.closed || (fabsf(p.x) < k.interior && fabsf(p.y) < k.interior));
   uint32_t mx[3];
 #pragma unroll
@@ -201,8 +196,12 @@ __device__ __forceinline__ uint32_t build_particle_list(const SppConsts& k, cons
                      : spp_pair_sep(&k, 0, p.x, p.y, q[u].x, q[u].y, &dx, &dy);
       }
 #pragma unroll
-      for (int u = 0; u < LIST_TRIP; ++u)
-        if (d2[u] < k.rlist2 && (int)j[u] != i) take(j[u]);
+      for (int u = 0; u < LIST_TRIP; ++u) {
+        const bool ok = d2[u] < k.rlist2 && (int)j[u] != i;
+        if (cnt < (uint32_t)LIST_LOCAL) col[cnt * stride] = j[u];   /* taken or overwritten: no lane waits */
+        else if (ok && cnt < cap) d.nbr[(size_t)cnt * d.n + i] = (int32_t)j[u];
+        cnt += ok;
+      }
     }
   }
   unsigned long long lane_cnt = 0;   /* neighbours per id % 4, 16 bits each */
