@@ -271,8 +271,8 @@ SWEEP_TOL = 0.02
 
 def point_alone(p, x, y, th, max_steps=20000):
     """One sweep point through the plain single-system path (System +
-    spp_step: the one-cluster kernel for small systems, the multi-kernel
-    step otherwise): max_steps steps, the stationary P = mean of P over the
+    spp_step: one resident launch per call where the system fits, the
+    multi-kernel step otherwise): max_steps steps, the stationary P = mean of P over the
     second half, sampled every step."""
     import numpy as np
     from spp_gb300 import System
@@ -337,7 +337,7 @@ def sweep_leg(sample_points=64, seed=4):
                            "sampled_points": int(len(sample)),
                            "sample": "seeded random sample stratified by N (equal counts per size quartile), "
                                      "each point run alone to 20,000 steps through System + spp_step (the "
-                                     "one-cluster kernel where the system fits, else the multi-kernel step), "
+                                     "resident run where the system fits, else the multi-kernel step), "
                                      "P every step over the second half; mean time per point x all points"},
         "speedup_vs_point_by_point": (int(within.sum()) / res.wall_s) / (1.0 / mean_pp),
         "speedup_vs_batched_plain": (int(within.sum()) / res.wall_s) / (n / plain.wall_s),
@@ -703,7 +703,8 @@ def other_workload(args):
                          "note": "effective bandwidth of the whole step; working set L2-resident"}}
     if w == "vesicles":
         line["roofline"]["traffic"] = ncu_traffic_per_launch(p.n, "k_abp_stage_vesicles163k_rk4.md")
-        line["roofline"]["traffic_note"] = "cold-cache DRAM bytes per k_abp_stage launch (ncu, 4 stages per step)"
+        line["roofline"]["traffic_note"] = ("cold-cache DRAM bytes per k_abp_stage launch (ncu, 4 stages per step), "
+                                            "the path of larger systems")
     line.update(extra)
     if not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_baseline_workload(w, unit)

@@ -168,8 +168,9 @@ __device__ __forceinline__ void segments(const DevBatch& b, const BatchSys* S, S
  * clears the counts (25 us instead of 90: k_scan_counts) and the bookkeeping
  * beside the scan: 504 / 822.  Row by row instead of the three rows flattened
  * into one sequence with comparisons for the image (about 20 instructions a
- * candidate -> 13): 479 / 674.  What bounds it: issue (78% of the slots), the
- * walk's loads, and warps that wait for their longest walk (28 of 32 lanes).
+ * candidate -> 13): 479 / 674.  What bounds it: issue (77% of the slots), the
+ * walk's loads, and lanes that wait for their warp's longest rows (22 of 32
+ * active).
  * Slower: blocks of 64 or 128 threads (less L1 reuse, 634 and 616 against 605
  * some 200 steps in), a second copy of the walk without the image shift (811:
  * spills), the rows as a rolled loop (617). */

@@ -20,7 +20,7 @@
  *
  * Measured on one GB300 (us per step, ABP at unit density; step graphs ->
  * resident): RK2 N = 16,384: 22 -> 8.6; RK2 N = 65,536: 23 -> 10.0; vesicles
- * (163,840 bodies, RK4): 38 -> 25.2.  A stage at N = 16,384 is about 6,300
+ * (163,840 bodies, RK4): 38 -> 22.1.  A stage at N = 16,384 is about 6,300
  * cycles: 1,700 for the gathers and pair terms, 1,250 for the update, 1,700
  * until the block's stores are visible and its arrival is out, 1,500 to
  * 2,000 for the other blocks' arrivals.  What bounds it is that chain of L2
