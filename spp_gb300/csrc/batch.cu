@@ -20,6 +20,7 @@
  * four moments over a start-up window, and its mean over a stationary
  * window -- the inputs and targets of the sweep surrogate.
  */
+#include <algorithm>
 #include <cmath>
 #include <cstddef>
 #include <cstring>
@@ -168,7 +169,8 @@ __device__ __forceinline__ void segments(const DevBatch& b, const BatchSys* S, S
  * clears the counts (25 us instead of 90: k_scan_counts) and the bookkeeping
  * beside the scan: 504 / 822.  Row by row instead of the three rows flattened
  * into one sequence with comparisons for the image (about 20 instructions a
- * candidate -> 13): 479 / 674.  What bounds it: issue (77% of the slots), the
+ * candidate -> 13): 479 / 674; systems ordered by expected flocks: 471 / 561.
+ * What bounds it: issue (77% of the slots), the
  * walk's loads, and lanes that wait for their warp's longest rows (22 of 32
  * active).
  * Slower: blocks of 64 or 128 threads (less L1 reuse, 634 and 616 against 605
@@ -423,15 +425,18 @@ void batch_free(SppBatch* b) {
  * Measured on one GB300 (us per batched step over the first 32 steps / after
  * 300, flocking):
  *   vector sum   <., 4, 5>        <., 2, 8>
- *     834k       68 / 148         64 / 154
- *     1.8M       145 / 239        138 / 227
- *     7.4M       538 / 722        479 / 672
+ *     834k       60 / 128         57 / 143
+ *     1.8M       138 / 176        130 / 192
+ *     3.6M       268 / 330        241 / 293
+ *     7.4M       540 / 650        479 / 567
  * Small batches wait on their longest walks, large ones want the warps.
- * Angles: <., 2, 8> 68 / 77 and 525 / 550 (834k, 7.4M), <., 4, 5> 69 / 75 and
- * 576 / 613.  The push needs registers: <., 1, 5> 105 / 496 and 827 / 1654,
- * <., 4, 5> 123 / 591 and 956 / 1979, <., 4, 4> 109 / 480 and 905 / 1769,
- * <., 1, 6> 127 / 637 and 987 / 2358; mixed batches the same order. */
-constexpr int BATCH_LARGE = 1500000;
+ * Angles: <., 2, 8> 63 / 66 and 525 / 552 (834k, 7.4M); <., 4, 5>, measured
+ * with the systems in the caller's order, 69 / 75 against 68 / 77 and 576 /
+ * 613 against 525 / 550.  The push needs registers: <., 1, 5> 90 / 432 and 811 /
+ * 1548, <., 2, 5> 95 / 464 and 853 / 1654, <., 4, 4> 96 / 407 and 897 / 1698;
+ * mixed batches the same order (82 / 205 and 720 / 1116, 92 / 241 and 796 /
+ * 1275, 92 / 198 and 839 / 1283). */
+constexpr int BATCH_LARGE = 2500000;
 
 /* One step, captured on st.  The per-system bookkeeping (k_batch_finish) runs
  * beside the next step's scan: it forks off after the step kernel and is
@@ -486,7 +491,21 @@ int batch_refresh_active(SppBatch* b) {
   std::vector<uint32_t> act_sys;
   act_sys.reserve((size_t)d.n_total);
   uint32_t a_poff = 0, a_coff = 0;
-  for (int s = 0; s < ns; ++s) {
+  /* Where flocks are to be expected first: their walks are the longest, and
+   * started last they would leave the GPU waiting for them.  Density over
+   * noise (noise alone comes close, density alone does not); us per step over the
+   * steps 300 to 332, in the caller's order / this: 64 points 149 / 128, 256
+   * points 348 / 292, 512 points 671 / 562; unflocked 68 / 60, 246 / 239, 483 /
+   * 472.  By size, largest first: 148, 357, 724. */
+  auto flocks = [&](int s) {
+    const BatchSys& S = b->host_sys[(size_t)s];
+    const float w = (float)S.n / ((float)S.D * (float)S.D * (S.k.eta + 0.01f));
+    return std::isfinite(w) ? w : 0.0f;
+  };
+  std::vector<int> order((size_t)ns);
+  for (int s = 0; s < ns; ++s) order[(size_t)s] = s;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return flocks(x) > flocks(y); });
+  for (int s : order) {
     const BatchSys& S = b->host_sys[(size_t)s];
     sact[(size_t)s] = {0u, 0};
     if (!flags[(size_t)s]) continue;
