@@ -170,16 +170,19 @@ constexpr int HIST_THREADS = 512;
 constexpr int HIST_LANES = 8;
 constexpr int HIST_CHUNK = HIST_THREADS / HIST_LANES;   /* particles */
 
-template <bool RADIAL>
+/* NEAR: the edges fit shared memory (a long thin body-frame grid's, past
+ * 58,000 bins on a side, do not; they are read from global memory). */
+template <bool RADIAL, bool NEAR>
 __global__ void __launch_bounds__(HIST_THREADS, 2) k_obs_hist(Grid g, HistArgs h, unsigned long long* counts) {
   extern __shared__ float hist_mem[];
-  float* const edges = hist_mem;                                        /* [nedges] */
-  uint32_t* const hist = reinterpret_cast<uint32_t*>(edges + h.nedges);  /* [nbins][copies] */
+  const float* const edges = NEAR ? hist_mem : h.edges;                 /* [nedges] */
+  uint32_t* const hist = reinterpret_cast<uint32_t*>(hist_mem + (NEAR ? h.nedges : 0));  /* [nbins][copies] */
   const int lane_copy = threadIdx.x & (h.copies - 1);
   const int words = h.local ? h.nbins * h.copies : 0;
   const int chunks = (g.n + HIST_CHUNK - 1) / HIST_CHUNK;
   for (int b = threadIdx.x; b < words; b += HIST_THREADS) hist[b] = 0u;
-  for (int b = threadIdx.x; b < h.nedges; b += HIST_THREADS) edges[b] = h.edges[b];
+  if (NEAR)
+    for (int b = threadIdx.x; b < h.nedges; b += HIST_THREADS) hist_mem[b] = h.edges[b];
   __syncthreads();
   auto add = [&](int b) {
     if (h.local) atomicAdd(&hist[b * h.copies + lane_copy], 1u);
@@ -416,6 +419,20 @@ int grid_build(SppSystem* s, double range, size_t nbins, size_t nedges, Grid* g,
   return SPP_OK;
 }
 
+/* The histogram of the grid's pairs into bins, with smem bytes of shared
+ * memory per block. */
+template <bool RADIAL, bool NEAR>
+int launch_hist(const Grid& g, const HistArgs& h, unsigned long long* bins, int sms, int most, size_t smem,
+                cudaStream_t st) {
+  OCUDA(cudaFuncSetAttribute(k_obs_hist<RADIAL, NEAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  int per_sm = 1;
+  OCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_obs_hist<RADIAL, NEAR>, HIST_THREADS, smem));
+  const int chunks = (g.n + HIST_CHUNK - 1) / HIST_CHUNK;
+  const int blocks = std::min(chunks, sms * std::max(per_sm, 1));
+  k_obs_hist<RADIAL, NEAR><<<blocks, HIST_THREADS, smem, st>>>(g, h, bins);
+  return SPP_OK;
+}
+
 /* The histogram of the grid's pairs into counts (host). */
 template <bool RADIAL>
 int run_hist(SppSystem* s, const Grid& g, HistArgs h, unsigned long long* bins, uint64_t* counts, cudaStream_t st) {
@@ -436,14 +453,12 @@ int run_hist(SppSystem* s, const Grid& g, HistArgs h, unsigned long long* bins, 
   if (chunk_most >= 4294967295.0) h.local = 0;
   h.per_flush = (int)std::fmin(1e6, std::floor(4294967295.0 / chunk_most));
   if (!h.local) h.copies = 1;
-  const size_t smem = fixed + (h.local ? h.copies * one : 0);
-  OCUDA(cudaFuncSetAttribute(k_obs_hist<RADIAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  int per_sm = 1;
-  OCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_obs_hist<RADIAL>, HIST_THREADS, smem));
-  const int chunks = (g.n + HIST_CHUNK - 1) / HIST_CHUNK;
-  const int blocks = std::min(chunks, sms * std::max(per_sm, 1));
+  const bool near = fixed <= (size_t)most;   /* a radial histogram's edges always are */
+  const size_t smem = (near ? fixed : 0) + (h.local ? h.copies * one : 0);
   k_obs_edges<RADIAL><<<nblk(h.nedges), SPP_BLOCK, 0, st>>>(h, const_cast<float*>(h.edges));
-  k_obs_hist<RADIAL><<<blocks, HIST_THREADS, smem, st>>>(g, h, bins);
+  const int rc = RADIAL || near ? launch_hist<RADIAL, true>(g, h, bins, sms, most, smem, st)
+                                : launch_hist<false, false>(g, h, bins, sms, most, smem, st);
+  if (rc != SPP_OK) return rc;
   spp_internal_count_launches(s, 2);
   OCUDA(cudaGetLastError());
   OCUDA(cudaMemcpyAsync(counts, bins, sizeof(uint64_t) * (size_t)h.nbins, cudaMemcpyDeviceToHost, st));

@@ -64,3 +64,16 @@ def test_radial_on_a_grid_of_many_cells(gpu_lib):
     with System(configs.vicsek_config(n=n, L=L)) as s:
         s.upload(x, y, np.zeros(n, np.float32))
         assert np.array_equal(s.radial_distribution(0.2, 7), want)
+
+
+@pytest.mark.parametrize("gx,gy", [(65536, 1), (1, 65536), (58109, 1), (58110, 1), (1, 58111)])
+def test_body_frame_on_a_thin_grid(gpu_lib, gx, gy):
+    """The most bins a grid may have, all on one side: more edges than shared
+    memory holds (and the last that it holds)."""
+    n, L = 500, 8.0
+    x, y, th = frame(n, L, 3)
+    c, sn = O.math32("cos", th), O.math32("sin", th)
+    with System(configs.vicsek_config(n=n, L=L)) as s:
+        s.upload(x, y, th)
+        got = s.pair_distribution(2.0, 1.5, gx, gy)
+    assert np.array_equal(got, O.pair_distribution32(x, y, c, sn, 2.0, 1.5, gx, gy))
