@@ -37,7 +37,6 @@ int fail(int status, const std::string& msg) {
   } while (0)
 
 constexpr int GRAPH_CHUNK = 32;
-constexpr int RUN_CHUNK = 1 << 14;   /* steps of one resident launch at most */
 
 /* A system's pinned host memory.  Copies to and from pageable memory wait
  * one by one inside the driver (about 10 us each); through this block a call
@@ -335,7 +334,7 @@ int enqueue_rebuild(SppSystem* s, cudaStream_t st, int64_t* launches) {
 /* One step of the model, enqueued on st (stream or capture). */
 int enqueue_step(SppSystem* s, cudaStream_t st, bool capture, int64_t* launches) {
   if (s->vrun.blocks > 0) {
-    if (launch_vrun(s->k, s->d, s->vrun, s->vbuf, 1, 0, nullptr, st) != 0)
+    if (launch_vrun(s->k, s->d, s->vrun, s->vbuf, 1, 0, 0, nullptr, st) != 0)
       return fail(SPP_ERR_CUDA, std::string("k_vrun: ") + cudaGetErrorString(cudaGetLastError()));
     if (launches) *launches += 1;
     return SPP_OK;
@@ -416,19 +415,16 @@ bool vicsek_captures(const SppSystem* s) {
   return n <= 16384 && cells < 65536 && per_particle * n + 8 * cells <= 224 * 1024;
 }
 
-/* nsteps steps of a resident Vicsek run, in launches of whole frames. */
+/* nsteps steps of a resident Vicsek run, with the heading sums of a frame
+ * after every `every` (0: no frames). */
 int run_vicsek(SppSystem* s, int64_t nsteps, int every, unsigned long long* sums) {
-  const int64_t unit = every > 0 ? every : 1;
-  const int64_t most = RUN_CHUNK / unit > 0 ? RUN_CHUNK / unit * unit : unit;
-  while (nsteps > 0) {
-    const int chunk = (int)(nsteps > most ? most : nsteps);
-    if (launch_vrun(s->k, s->d, s->vrun, s->vbuf, chunk, every, sums, s->stream) != 0)
+  return spp_for_parts(nsteps, every, [&](const RunPart& q) {
+    if (launch_vrun(s->k, s->d, s->vrun, s->vbuf, q.steps, q.first, every, sums, s->stream) != 0)
       return fail(SPP_ERR_CUDA, std::string("k_vrun: ") + cudaGetErrorString(cudaGetLastError()));
     s->host_launches++;
-    if (sums) sums += 2 * (chunk / unit);
-    nsteps -= chunk;
-  }
-  return SPP_OK;
+    if (sums) sums += 2 * q.events;
+    return (int)SPP_OK;
+  });
 }
 
 int run_steps(SppSystem* s, int64_t nsteps) {
@@ -460,13 +456,13 @@ int run_steps(SppSystem* s, int64_t nsteps) {
     /* a stream that is being captured takes the graph path, which refuses it */
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CUDA_TRY(cudaStreamIsCapturing(s->stream, &cs));
-    while (cs == cudaStreamCaptureStatusNone && nsteps > 0) {
-      const int chunk = nsteps > RUN_CHUNK ? RUN_CHUNK : (int)nsteps;
-      if (launch_run(s->k, s->d, s->run, s->nstages, chunk, s->stream) != 0)
-        return fail(SPP_ERR_CUDA, std::string("k_run: ") + cudaGetErrorString(cudaGetLastError()));
-      s->graph_kernels += (int64_t)chunk * s->per_step_kernels;
-      nsteps -= chunk;
-    }
+    if (cs == cudaStreamCaptureStatusNone)
+      return spp_for_parts(nsteps, 0, [&](const RunPart& q) {
+        if (launch_run(s->k, s->d, s->run, s->nstages, q.steps, s->stream) != 0)
+          return fail(SPP_ERR_CUDA, std::string("k_run: ") + cudaGetErrorString(cudaGetLastError()));
+        s->graph_kernels += (int64_t)q.steps * s->per_step_kernels;
+        return (int)SPP_OK;
+      });
   }
   while (nsteps > 0) {
     int chunk = nsteps >= GRAPH_CHUNK ? GRAPH_CHUNK : (int)nsteps;
@@ -693,15 +689,15 @@ int launch_lyap_chunks(SppSystem* s, int64_t nsteps) {
   if (s->lrun.blocks > 0) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CUDA_TRY(cudaStreamIsCapturing(s->stream, &cs));
-    const int64_t most = RUN_CHUNK / every > 0 ? (int64_t)(RUN_CHUNK / every) * every : every;
-    while (cs == cudaStreamCaptureStatusNone && left > 0) {
-      const int part = (int)(left > most ? most : left);
-      if (launch_lrun(s->k, s->d, s->lyap, s->lrun, s->nstages, part, every, s->stream) != 0)
-        return fail(SPP_ERR_CUDA, std::string("k_lrun: ") + cudaGetErrorString(cudaGetLastError()));
-      /* the passes that the step graphs would launch */
-      s->graph_kernels += (int64_t)part * (2 * s->nstages + 1) + 6 * ((part + every - 1) / every);
-      left -= part;
-    }
+    if (cs == cudaStreamCaptureStatusNone)
+      return spp_for_parts(left, every, [&](const RunPart& q) {
+        if (launch_lrun(s->k, s->d, s->lyap, s->lrun, s->nstages, q.steps, q.first, every, q.last, s->stream) != 0)
+          return fail(SPP_ERR_CUDA, std::string("k_lrun: ") + cudaGetErrorString(cudaGetLastError()));
+        /* the passes that the step graphs would launch */
+        const int renorms = q.events + (q.last && spp_next_event(q.steps, q.first, every) != every);
+        s->graph_kernels += (int64_t)q.steps * (2 * s->nstages + 1) + 6 * renorms;
+        return (int)SPP_OK;
+      });
   }
   while (left > 0) {
     int chunk = left >= every ? every : (int)left;

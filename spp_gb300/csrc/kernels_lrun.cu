@@ -191,11 +191,12 @@ __device__ __noinline__ bool lrun_renormalize(const DevState& d, const LyapState
   return true;
 }
 
-/* nsteps steps, renormalised after every `every` and after the last. */
+/* nsteps steps, renormalised after the steps first, first + every, ... and,
+ * with finish, after the last. */
 template <int LANES, int KP>
 __global__ void __launch_bounds__(lrun_threads(LANES), 1)
     k_lrun(const __grid_constant__ SppConsts k, const __grid_constant__ DevState d, const __grid_constant__ LyapState L,
-           int nst, int nsteps, int every) {
+           int nst, int nsteps, int first, int every, bool finish) {
   constexpr int VPL = KP / LANES;          /* vectors per lane: v = lane_r + LANES m */
   constexpr int GROUP = LANES == 1 ? 3 : 2;   /* neighbours gathered together */
   constexpr int BIG = 3;                      /* the same for long segments */
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
   const float gp = k.g * k.one_minus_alpha_over_pi;
   if (!barrier()) return;
 
-  int to_renorm = every;
+  int to_renorm = first;
   int t = 0;
   for (; t < nsteps && !frozen; ++t) {
     const float x0 = p.x, y0 = p.y;
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
     }
     ++step;
     const bool rebuild = decision & 2u;
-    const bool renorm = --to_renorm == 0 || t + 1 == nsteps;
+    const bool renorm = --to_renorm == 0 || (finish && t + 1 == nsteps);
     if (!rebuild && !renorm) continue;
     store_vectors();
     if (rebuild) {
@@ -553,12 +554,15 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
   }
   if (frozen) {
     /* a list overflowed: as in the step graphs, whose stages skip the steps
-     * left but whose renormalisations run, one for every chunk of `every`
-     * steps from that of the last good step on; the vectors are in L.t0 */
+     * left but whose renormalisations run, from that of the last good step on;
+     * the vectors are in L.t0 */
     if (!barrier()) return;
-    const int chunks = (nsteps + every - 1) / every;
-    for (int c = t > 0 ? (t - 1) / every : 0; c < chunks; ++c)
+    const int done = t > 0 ? spp_events_upto(t - 1, first, every) : 0;
+    const int all = spp_events_upto(nsteps, first, every) + (finish && spp_next_event(nsteps, first, every) != every);
+    for (int c = done; c < all; ++c)
       if (!lrun_renormalize<KP>(d, L, &target, &s_word, &chol, warp_part)) return;
+  } else {
+    store_vectors();   /* those of a launch that ends between renormalisations */
   }
 
   if (head) {
@@ -580,7 +584,7 @@ __global__ void __launch_bounds__(lrun_threads(LANES), 1)
   }
 }
 
-typedef void (*LrunKernel)(SppConsts, DevState, LyapState, int, int, int);
+typedef void (*LrunKernel)(SppConsts, DevState, LyapState, int, int, int, int, bool);
 
 LrunKernel lrun_kernel(int lanes, int K) {
   if (lanes == SPP_GATHER_LANES) return K <= 4 ? (LrunKernel)k_lrun<4, 4> : (LrunKernel)k_lrun<4, 8>;
@@ -621,7 +625,7 @@ bool plan_lrun(const SppConsts& k, const DevState& d, int K, RunPlan* plan) {
 }
 
 int launch_lrun(const SppConsts& k, const DevState& d, const LyapState& L, const RunPlan& plan, int nstages, int nsteps,
-                int every, cudaStream_t s) {
+                int first, int every, bool finish, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -632,5 +636,8 @@ int launch_lrun(const SppConsts& k, const DevState& d, const LyapState& L, const
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, lrun_kernel(k.lanes, L.K), k, d, L, nstages, nsteps, every) == cudaSuccess ? 0 : -1;
+  return cudaLaunchKernelEx(&cfg, lrun_kernel(k.lanes, L.K), k, d, L, nstages, nsteps, first, every, finish) ==
+                 cudaSuccess
+             ? 0
+             : -1;
 }

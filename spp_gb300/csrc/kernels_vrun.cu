@@ -82,7 +82,7 @@ __device__ __forceinline__ void vrun_pair(const SppConsts& k, VrunAcc* acc, floa
 template <int MODEL, int LANES, int PER_SM>
 __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
     k_vrun(const __grid_constant__ SppConsts k, const __grid_constant__ DevState d, const __grid_constant__ VrunBufs vb,
-           int nsteps, int every, unsigned long long* sums) {
+           int nsteps, int first, int every, unsigned long long* sums) {
   constexpr bool ANGLE = MODEL == SPP_MODEL_VICSEK_REF_ANGLE;
   constexpr int NC = (9 + LANES - 1) / LANES;   /* cells per lane */
   constexpr int AT_ONCE = 3;                    /* cells whose loads are issued together */
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
   uint32_t word = head ? spp_draw_k(&k, pid, step, SPP_RNG_VICSEK).v[0] : 0u;
   if (!barrier()) return;
 
-  int to_frame = every;
+  int to_frame = first;
   for (int t = 0; t < nsteps; ++t, ++step) {
     {
       uint32_t* const clear = vb.count[(t + 2) % 3];
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
   }
 }
 
-typedef void (*VrunKernel)(SppConsts, DevState, VrunBufs, int, int, unsigned long long*);
+typedef void (*VrunKernel)(SppConsts, DevState, VrunBufs, int, int, int, unsigned long long*);
 
 template <int MODEL>
 VrunKernel vrun_kernel_for(int lanes, int per_sm) {
@@ -428,8 +428,8 @@ bool plan_vrun(const SppConsts& k, const DevState& d, VrunPlan* plan) {
   return cells * plan->cap * 2 * sizeof(float4) <= (1ull << 30);
 }
 
-int launch_vrun(const SppConsts& k, const DevState& d, const VrunPlan& plan, const VrunBufs& vb, int nsteps, int every,
-                unsigned long long* sums, cudaStream_t s) {
+int launch_vrun(const SppConsts& k, const DevState& d, const VrunPlan& plan, const VrunBufs& vb, int nsteps, int first,
+                int every, unsigned long long* sums, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -439,7 +439,7 @@ int launch_vrun(const SppConsts& k, const DevState& d, const VrunPlan& plan, con
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, vrun_kernel(k.model, plan.lanes, plan.per_sm), k, d, vb, nsteps, every, sums) ==
+  return cudaLaunchKernelEx(&cfg, vrun_kernel(k.model, plan.lanes, plan.per_sm), k, d, vb, nsteps, first, every, sums) ==
                  cudaSuccess
              ? 0
              : -1;

@@ -21,6 +21,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "spp_parts.h"
 #include "spp_physics.h"
 
 #define SPP_BLOCK 256
@@ -159,7 +160,6 @@ void launch_abp_stage(const SppConsts& k, const DevState& d, int stage, int nsta
 /* kernels_run.cu: nsteps whole steps of a Verlet-list system in one
  * cooperative launch.  plan_run: whether the system fits (every thread of
  * its neighbour sums resident at once) and the launch shape. */
-#define RUN_MAX_BLOCKS 1024
 struct RunPlan {
   int blocks, threads;    /* 0: the system does not fit */
   int per_sm;             /* blocks per SM the kernel is compiled for (1 or 2) */
@@ -167,8 +167,8 @@ struct RunPlan {
 bool plan_run(const SppConsts& k, const DevState& d, RunPlan* plan);
 int launch_run(const SppConsts& k, const DevState& d, const RunPlan& plan, int nstages, int nsteps, cudaStream_t s);
 /* kernels_vrun.cu: the same for the discrete Vicsek models.  every > 0: the
- * fixed-point heading sums after every `every` steps are added into sums
- * (two words per frame, zeroed by the caller). */
+ * fixed-point heading sums after the steps first, first + every, ... are added
+ * into sums (two words per frame, zeroed by the caller). */
 struct VrunPlan {
   int blocks, threads;    /* 0 blocks: the system does not fit */
   int lanes, per_sm;
@@ -184,8 +184,8 @@ struct VrunBufs {
   int cap;
 };
 bool plan_vrun(const SppConsts& k, const DevState& d, VrunPlan* plan);
-int launch_vrun(const SppConsts& k, const DevState& d, const VrunPlan& plan, const VrunBufs& vb, int nsteps, int every,
-                unsigned long long* sums, cudaStream_t s);
+int launch_vrun(const SppConsts& k, const DevState& d, const VrunPlan& plan, const VrunBufs& vb, int nsteps, int first,
+                int every, unsigned long long* sums, cudaStream_t s);
 void launch_vicsek_step(const SppConsts& k, const DevState& d, cudaStream_t s, int64_t* launches);
 void launch_polarization(const DevState& d, cudaStream_t s);
 /* the two fixed-point heading sums added into sums[0..1] (zeroed by the caller) */

@@ -30,10 +30,11 @@ struct TanStage {
 void launch_tangent_stage(const SppConsts& k, const DevState& d, const LyapState& L, int stage,
                           int nstages, const float4* cur, cudaStream_t s, int64_t* launches);
 /* kernels_lrun.cu: nsteps steps of base and tangent dynamics in one
- * cooperative launch, renormalised after every `every` steps and at the end */
+ * cooperative launch, renormalised after the steps first, first + every, ...
+ * and, with finish, after the last */
 bool plan_lrun(const SppConsts& k, const DevState& d, int K, RunPlan* plan);
 int launch_lrun(const SppConsts& k, const DevState& d, const LyapState& L, const RunPlan& plan, int nstages, int nsteps,
-                int every, cudaStream_t s);
+                int first, int every, bool finish, cudaStream_t s);
 void launch_renormalize(const LyapState& L, int accumulate, cudaStream_t s, int64_t* launches);
 void launch_tangent_init(const LyapState& L, uint64_t seed, uint32_t system, cudaStream_t s);
 /* floats of LyapState::uslot for K vectors of n particles */
