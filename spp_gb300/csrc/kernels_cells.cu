@@ -185,8 +185,7 @@ __global__ void __launch_bounds__(SPP_BLOCK, 6) k_build_list(SppConsts k, DevSta
 }
 
 /* Lists longer than LIST_LOCAL, queued by k_build_list: one warp per list
- * (grid-stride over the queue).  Lists beyond 512 entries, which only
- * extreme densities produce, are insertion-sorted by one lane. */
+ * (grid-stride over the queue). */
 __global__ void __launch_bounds__(SPP_BLOCK) k_sort_long(SppConsts k, DevState d) {
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);

@@ -306,20 +306,42 @@ __device__ __forceinline__ void warp_sort_list(const SppConsts& k, const DevStat
   }
 }
 
-/* The list of particle i (m entries) insertion-sorted in place by one
- * thread: lists beyond 512 entries, which only extreme densities produce. */
-__device__ __forceinline__ void insertion_sort_list(const SppConsts& k, const DevState& d, int i, int m) {
-  for (int q = 1; q < m; ++q) {
-    const int32_t j = d.nbr[(size_t)q * d.n + i];
-    const uint32_t oj = spp_list_order(&k, d.id_alt[j]);
-    int pos = q;
-    while (pos > 0) {
-      const int32_t prev = d.nbr[(size_t)(pos - 1) * d.n + i];
-      if (spp_list_order(&k, d.id_alt[prev]) < oj) break;
-      d.nbr[(size_t)pos * d.n + i] = prev;
-      --pos;
+/* The list of particle i (m entries) sorted in place by the calling warp:
+ * lists beyond 512 entries, which only clumps produce.  Batcher's bitonic
+ * sorter for any m: a merge of runs compares mirrored places first, then
+ * places a stride apart, always ascending, so the places from m on, which
+ * hold the largest keys, never exchange.  A resident run does this between
+ * grid barriers that give up after seconds, so the time has to be bounded: a
+ * list of 5,000 takes 91 passes of 128 comparisons per lane (an insertion by
+ * one lane took 6 million dependent loads, some seconds). */
+__device__ __forceinline__ void sort_list_in_place(const SppConsts& k, const DevState& d, int i, int m) {
+  const int lane = threadIdx.x & 31;
+  auto exchange = [&](int lo, int hi) {
+    if (hi >= m) return;
+    int32_t* const a = d.nbr + (size_t)lo * d.n + i;
+    int32_t* const b = d.nbr + (size_t)hi * d.n + i;
+    const int32_t ja = *a, jb = *b;
+    if (!spp_index_ok(d.ctl, ja, d.n) || !spp_index_ok(d.ctl, jb, d.n)) return;
+    if (spp_list_order(&k, d.id_alt[ja]) > spp_list_order(&k, d.id_alt[jb])) {
+      *a = jb;
+      *b = ja;
     }
-    d.nbr[(size_t)pos * d.n + i] = j;
+  };
+  int size = 2;
+  while (size < m) size <<= 1;
+  for (int run = 2; run <= size; run <<= 1) {
+    for (int e = lane; e < size / 2; e += 32) {
+      const int at = e / (run / 2) * run, o = e % (run / 2);
+      exchange(at + o, at + run - 1 - o);
+    }
+    __syncwarp();
+    for (int stride = run >> 2; stride > 0; stride >>= 1) {
+      for (int e = lane; e < size / 2; e += 32) {
+        const int lo = 2 * e - (e & (stride - 1));
+        exchange(lo, lo + stride);
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -332,7 +354,7 @@ __device__ __forceinline__ void sort_queued_list(const SppConsts& k, const DevSt
   else if (m <= 128) warp_sort_list<4>(k, d, i, m);
   else if (m <= 256) warp_sort_list<8>(k, d, i, m);
   else if (m <= 512) warp_sort_list<16>(k, d, i, m);
-  else if ((threadIdx.x & 31) == 0) insertion_sort_list(k, d, i, m);
+  else sort_list_in_place(k, d, i, m);
 }
 
 }  // namespace

@@ -31,7 +31,7 @@ __device__ __forceinline__ void run_sort_list(const SppConsts& k, const DevState
   const int lane = threadIdx.x & 31;
   const int m = d.nn[i];
   if (m > RUN_SORT_MAX) {
-    if (lane == 0) insertion_sort_list(k, d, i, m);
+    sort_list_in_place(k, d, i, m);
     return;
   }
   int size = 32;
