@@ -1039,6 +1039,7 @@ int spp_upload_state(SppSystem* s, const float* x, const float* y, const float* 
   Ctl c;
   memset(&c, 0, sizeof(c));
   c.step = (uint32_t)step0;
+  c.run_sorted = (uint32_t)step0;
   c.bad_nonfinite = 0xffffffffu;
   c.bad_range = 0xffffffffu;
   s->host->ctl = c;

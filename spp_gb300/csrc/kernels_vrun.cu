@@ -14,9 +14,9 @@
  * that of the multi-kernel step (k_bin_count / scan / k_scatter /
  * k_vicsek_step) bit for bit.
  *
- * Every VRUN_SORT steps the particles change hands in cell order (a scan of
- * the counts, a scatter, three barriers), so that a warp's threads read the
- * same cells.  A step in which some cell holds more than the bucket's
+ * Every RUN_SORT_STEPS steps, over calls, the particles change hands in cell
+ * order (a scan of the counts, a scatter, three barriers), so that a warp's
+ * threads read the same cells.  A step in which some cell holds more than the bucket's
  * capacity (flocks) does the same and takes its candidates from the sorted
  * copy; the run stays in this kernel.
  *
@@ -35,7 +35,9 @@
  * 21.9 / 20.0 and 49.6 / 44.3 / 39.8; the other rules, whose terms need the
  * registers: angles at 50,001 15.9 / 15.7 / 16.7, push 59 / 56 / 55.
  * Without the sorts N = 50,001 took 28.4 (17.0 with them at the time), with
- * one every 8 steps as long as with one every 16.
+ * one every 8 steps as long as with one every 16.  Counted over calls (calls of
+ * 16 steps at N = 4,097 / 50,001 / 120,001: 6.6 / 16.7 / 25.3 us when every call
+ * counted for itself, 6.1 / 13.9 / 22.4 now; calls of 100: 5.6 / 13.4 / 21.8).
  */
 #include "spp_internal.cuh"
 #include "spp_grid.cuh"
@@ -45,8 +47,6 @@
 namespace {
 
 __host__ __device__ constexpr int vrun_threads(int per_sm) { return per_sm == 1 ? 640 : 576; }
-
-constexpr uint32_t VRUN_SORT = 16;   /* steps between two sorts of the owners */
 
 /* A bucket entry: position, and the packed parts of cos and sin. */
 __device__ __forceinline__ float pack_fx(float v) { return pack_parts(fx_parts(v)); }
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
   const bool inb = i < n;
   const bool head = inb && lane_r == 0;
   if (ctl->run_timeout) return;   /* the same for every block */
-  uint32_t step = ctl->step;
+  uint32_t step = ctl->step, sorted = ctl->run_sorted;
   unsigned target = 0;
   auto barrier = [&]() -> bool {
     target += gridDim.x;
@@ -162,7 +162,8 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
     }
     const uint32_t* const count = vb.count[t % 3];
     const unsigned full = *(volatile const unsigned*)(vb.full + t % 3);   /* the same for every thread of the grid */
-    if (full || (t > 0 && step % VRUN_SORT == 0)) {
+    if (full || spp_sort_due(step, sorted)) {
+      sorted = step;
       /* the particles change hands in cell order, so that a warp's threads
        * read the same cells; with a full bucket the step's candidates come
        * from this copy */
@@ -353,6 +354,7 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
   if (tid == 0) {
     if (blockIdx.x == 0) {
       ctl->step = step;
+      ctl->run_sorted = sorted;
       ctl->need_rebuild = 0u;
     }
     /* the last block to leave clears the barrier for the next launch */

@@ -49,7 +49,8 @@ struct Ctl {
   uint32_t run_disp[3], run_step[3];
   uint32_t run_exit;
   uint32_t run_timeout;
-  uint32_t pad0[32];
+  uint32_t run_sorted;    /* step at which a resident Vicsek run last put its owners in cell order */
+  uint32_t pad0[31];
   uint32_t run_bar;
   uint32_t pad1[31];
 };

@@ -23,6 +23,12 @@ SPP_HD int spp_next_event(int x, int first, int every) {
   return x < first ? first - x : every - (x - first) % every;
 }
 
+/* A resident Vicsek run puts its owners in cell order RUN_SORT_STEPS steps after
+ * the last time, counted over calls (Ctl.run_sorted): calls of 16 steps that
+ * counted for themselves would keep the order of the upload for ever. */
+#define RUN_SORT_STEPS 16u
+SPP_HD bool spp_sort_due(uint32_t step, uint32_t sorted) { return step - sorted >= RUN_SORT_STEPS; }
+
 struct RunPart {
   int steps;    /* of this launch */
   int first;    /* its step that ends with the first event (may lie beyond it); 0: no events */

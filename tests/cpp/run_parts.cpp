@@ -7,6 +7,9 @@ int run_chunk() { return RUN_CHUNK; }
 int run_arrivals() { return RUN_ARRIVALS; }
 int run_max_blocks() { return RUN_MAX_BLOCKS; }
 
+int sort_steps() { return (int)RUN_SORT_STEPS; }
+int sort_due(uint32_t step, uint32_t sorted) { return spp_sort_due(step, sorted); }
+
 // out: four words per launch (steps, first, events, last); the launches, or -1
 // once there are more than `room`.
 int parts(int64_t nsteps, int every, int32_t* out, int room) {

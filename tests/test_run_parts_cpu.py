@@ -1,7 +1,8 @@
 """How a call's steps are cut into resident launches (spp_parts.h): no launch is
 longer than its bound, whatever the distance between frames or
 renormalisations (so the grid barrier's 32-bit arrival count cannot wrap), and
-every event falls into one launch, at its step."""
+every event falls into one launch, at its step.  And when the owners of a
+resident Vicsek run are put in order again, whatever the length of the calls."""
 import ctypes as C
 import shutil
 import subprocess
@@ -23,6 +24,7 @@ def lib(tmp_path_factory):
                         str(SRC), "-o", str(so)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     lib = C.CDLL(str(so))
+    lib.sort_due.argtypes = [C.c_uint32, C.c_uint32]
     lib.parts.argtypes = [C.c_int64, C.c_int, C.POINTER(C.c_int32), C.c_int]
     return lib
 
@@ -60,3 +62,20 @@ def test_frames_further_apart_than_the_barrier_counts(lib):
     got = parts(lib, 1 << 31, 1 << 30)
     assert max(q[0] for q in got) * lib.run_arrivals() * lib.run_max_blocks() < 1 << 31
     assert sum(q[2] for q in got) == 2
+
+
+@pytest.mark.parametrize("start", [0, 5, (1 << 32) - 600])
+@pytest.mark.parametrize("calls", [1, 2, 3, 4, 8, 15, 16, 17, 32, 100])
+def test_owners_are_sorted_again_over_calls(lib, start, calls):
+    """A launch sorts before the first of its steps at which the rule says so;
+    the word that it reads is carried from call to call."""
+    sorted_at, last, gaps = start, start, []
+    step = start
+    while step < start + 500:
+        for _ in range(calls):
+            if lib.sort_due(step, sorted_at):
+                sorted_at = step
+                gaps.append(step - last)
+                last = step
+            step += 1
+    assert gaps and set(gaps) == {lib.sort_steps()}
