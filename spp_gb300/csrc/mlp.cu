@@ -585,7 +585,7 @@ __global__ void k_mlp_cast(int count, const float* master, __nv_bfloat16* w) {
 /* ------------------------------------------------------------------ */
 /* whole training runs: one thread-block cluster per ensemble member     */
 /* ------------------------------------------------------------------ */
-/* k_mlp_train runs every iteration of a training call in one launch.  The
+/* k_mlp_train runs many iterations of a training call in one launch.  The
  * members are independent, so each is one cluster of 16 CTAs, and the only
  * synchronisation is two hardware cluster barriers per iteration:
  *   A  the CTAs share the tiles of 16 samples, two at a time (eight warps
@@ -597,7 +597,7 @@ __global__ void k_mlp_cast(int count, const float* master, __nv_bfloat16* w) {
  *      warp per 16 x 8 entries), the other eight the remaining parameters of
  *      8 hidden units (the sums of k_mlp_grad_small); each parameter's Adam
  *      step follows at once.  Masters and moments stay with their owners (W2
- *      in registers, the others in shared memory) until the last iteration
+ *      in registers, the others in shared memory) until the launch's last iteration
  *      writes them back; the BF16 weights the next iteration reads are
  *      published through `pub` (16-byte aligned).
  * Every sum keeps the order of the kernels named above, so the trained
@@ -1245,6 +1245,17 @@ bool train_cluster_fits(int in) {
   return fits;
 }
 
+/* Iterations x samples x members of one launch at most, the time of an
+ * iteration being that of TRAIN_MIN_B samples and TRAIN_MIN_E members where
+ * there are fewer: 4 to 7 ms.  The training holds its SMs for the whole
+ * launch, so this is how long a call on another stream may wait (ms beside a
+ * long training of 5 members x 300 samples, 20 steps of a Vicsek system of
+ * 50,001, the training in one launch / this load / four times it: all of the
+ * training / 7 / 27; 100 steps of 300,000 disks beside 16 x 4,000: 53 / 10 / 14).
+ * A call of 300 iterations at 5 x 300 is one launch. */
+constexpr int64_t TRAIN_LOAD = 500000;
+constexpr int TRAIN_MIN_B = 300, TRAIN_MIN_E = 5;
+
 bool train_in_cluster(const SppMlp* m, int B) { return m->tensor_cores && m->train_cluster; }
 
 int mlp_train_cluster(SppMlp* m, int B, int iters, float lr) {
@@ -1257,8 +1268,6 @@ int mlp_train_cluster(SppMlp* m, int B, int iters, float lr) {
   a.vel = m->vel;
   a.w = m->w;
   a.pub = m->pub;
-  a.bias = m->bias;
-  a.iters = iters;
   a.lr = lr;
   a.b1 = ADAM_B1;
   a.b2 = ADAM_B2;
@@ -1275,7 +1284,13 @@ int mlp_train_cluster(SppMlp* m, int B, int iters, float lr) {
   cfg.stream = m->stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  MCUDA(cudaLaunchKernelEx(&cfg, k_mlp_train, a));
+  const int64_t load = (int64_t)(B > TRAIN_MIN_B ? B : TRAIN_MIN_B) * (m->E > TRAIN_MIN_E ? m->E : TRAIN_MIN_E);
+  const int most = TRAIN_LOAD / load > 0 ? (int)(TRAIN_LOAD / load) : 1;
+  for (int done = 0; done < iters; done += a.iters) {
+    a.bias = m->bias + done;
+    a.iters = iters - done < most ? iters - done : most;
+    MCUDA(cudaLaunchKernelEx(&cfg, k_mlp_train, a));
+  }
   return SPP_OK;
 }
 
