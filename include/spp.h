@@ -393,6 +393,9 @@ int spp_mlp_grad(SppMlp* m, const float* x, const float* t, const float* weights
  * last step. */
 int spp_mlp_train(SppMlp* m, const float* x, const float* t, const float* weights, int B, int iters, float lr,
                   float* loss);
+/* Launches so far that ran many training iterations each (a cluster of thread
+ * blocks per member); 0 where training runs as graphs of single iterations. */
+int64_t spp_mlp_resident_launches(SppMlp* m);
 
 /* ---- tangent-space Lyapunov spectrum (continuous model) ----
  * Replaces LyapunovBox (parallel/lyapunovbox.h:11-28): Init_Deviation
@@ -476,11 +479,15 @@ typedef struct SppTuneReport {
 } SppTuneReport;
 int spp_autotune(SppParams* p, const float* x, const float* y, const float* theta, int trial_steps,
                  int what, SppTuneReport* report);
-/* Number of kernels this handle has launched.  Graph replays count each
- * kernel node they run; a resident run (many steps of a small or mid-sized
- * Verlet-list system in one cooperative launch) counts the same stage and
- * rebuild passes that a replay of its steps would have launched. */
+/* Kernel passes this handle has run.  Graph replays count each kernel node
+ * they run; a resident run (many steps of a small or mid-sized system in one
+ * cooperative launch: spp_step, spp_lyap_step, spp_polarization_series) counts
+ * the passes that the step graphs would have launched for its steps, rebuilds
+ * and renormalisations. */
 int64_t spp_kernel_launches(SppSystem* s);
+/* Resident runs launched so far: their launches, each counted once.  0 for a
+ * system that steps through graphs. */
+int64_t spp_resident_launches(SppSystem* s);
 /* The cudaStream_t the handle launches on. */
 void* spp_stream(SppSystem* s);
 

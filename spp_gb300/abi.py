@@ -166,6 +166,7 @@ PROTOTYPES = {
     "spp_pairs": (C.c_int, [_P, C.c_double, _I32, _I32, C.c_int, C.POINTER(C.c_int64)]),
     "spp_cells": (C.c_int, [_P, C.c_int, C.c_int, _I32, _I32, C.c_int]),
     "spp_kernel_launches": (C.c_int64, [_P]),
+    "spp_resident_launches": (C.c_int64, [_P]),
     "spp_stream": (_P, [_P]),
     "spp_profile": (C.c_int, [_P, C.c_int, C.POINTER(SppProfile)]),
     "spp_time_steps": (C.c_int, [_P, C.c_int, C.POINTER(C.c_double)]),
@@ -195,6 +196,7 @@ PROTOTYPES = {
     "spp_mlp_predict": (C.c_int, [_P, _F, C.c_int, _F]),
     "spp_mlp_grad": (C.c_int, [_P, _F, _F, _F, C.c_int, _F, _F]),
     "spp_mlp_train": (C.c_int, [_P, _F, _F, _F, C.c_int, C.c_int, C.c_float, _F]),
+    "spp_mlp_resident_launches": (C.c_int64, [_P]),
     "spp_lyap_init": (C.c_int, [_P, C.c_int, C.c_uint64]),
     "spp_lyap_set_vectors": (C.c_int, [_P, _F, C.c_int]),
     "spp_lyap_step": (C.c_int, [_P, C.c_int, C.c_int]),

@@ -79,6 +79,7 @@ struct SppSystem {
   int per_rebuild_kernels = 0;
   int64_t host_launches = 0;
   int64_t graph_kernels = 0;
+  int64_t resident_launches = 0; /* k_run, k_vrun, k_lrun */
   int64_t direct_rebuilds = 0;
   int64_t regrowths = 0;         /* neighbour-list regrowths after an overflow */
   /* frame marked for spp_ring_motion: unwrapped positions and headings by
@@ -336,7 +337,8 @@ int enqueue_step(SppSystem* s, cudaStream_t st, bool capture, int64_t* launches)
   if (s->vrun.blocks > 0) {
     if (launch_vrun(s->k, s->d, s->vrun, s->vbuf, 1, 0, 0, nullptr, st) != 0)
       return fail(SPP_ERR_CUDA, std::string("k_vrun: ") + cudaGetErrorString(cudaGetLastError()));
-    if (launches) *launches += 1;
+    s->resident_launches++;
+    if (launches) *launches += s->per_step_kernels;
     return SPP_OK;
   }
   if (!s->uses_list) {
@@ -421,7 +423,9 @@ int run_vicsek(SppSystem* s, int64_t nsteps, int every, unsigned long long* sums
   return spp_for_parts(nsteps, every, [&](const RunPart& q) {
     if (launch_vrun(s->k, s->d, s->vrun, s->vbuf, q.steps, q.first, every, sums, s->stream) != 0)
       return fail(SPP_ERR_CUDA, std::string("k_vrun: ") + cudaGetErrorString(cudaGetLastError()));
-    s->host_launches++;
+    s->resident_launches++;
+    /* the passes that the step graphs would launch */
+    s->graph_kernels += (int64_t)q.steps * s->per_step_kernels + q.events;
     if (sums) sums += 2 * q.events;
     return (int)SPP_OK;
   });
@@ -460,6 +464,7 @@ int run_steps(SppSystem* s, int64_t nsteps) {
       return spp_for_parts(nsteps, 0, [&](const RunPart& q) {
         if (launch_run(s->k, s->d, s->run, s->nstages, q.steps, s->stream) != 0)
           return fail(SPP_ERR_CUDA, std::string("k_run: ") + cudaGetErrorString(cudaGetLastError()));
+        s->resident_launches++;
         s->graph_kernels += (int64_t)q.steps * s->per_step_kernels;
         return (int)SPP_OK;
       });
@@ -693,7 +698,7 @@ int launch_lyap_chunks(SppSystem* s, int64_t nsteps) {
       return spp_for_parts(left, every, [&](const RunPart& q) {
         if (launch_lrun(s->k, s->d, s->lyap, s->lrun, s->nstages, q.steps, q.first, every, q.last, s->stream) != 0)
           return fail(SPP_ERR_CUDA, std::string("k_lrun: ") + cudaGetErrorString(cudaGetLastError()));
-        /* the passes that the step graphs would launch */
+        s->resident_launches++;
         const int renorms = q.events + (q.last && spp_next_event(q.steps, q.first, every) != every);
         s->graph_kernels += (int64_t)q.steps * (2 * s->nstages + 1) + 6 * renorms;
         return (int)SPP_OK;
@@ -1460,6 +1465,8 @@ int64_t spp_kernel_launches(SppSystem* s) {
   if (graph_rebuilds < 0) graph_rebuilds = 0;
   return s->host_launches + s->graph_kernels + graph_rebuilds * s->per_rebuild_kernels;
 }
+
+int64_t spp_resident_launches(SppSystem* s) { return s ? s->resident_launches : 0; }
 
 void* spp_stream(SppSystem* s) { return s ? (void*)s->stream : nullptr; }
 

@@ -1078,6 +1078,7 @@ struct SppMlp {
   std::vector<TrainGraph> graphs;
   __nv_bfloat16* pub = nullptr;   /* weights as k_mlp_train reads them */
   bool train_cluster = false;     /* k_mlp_train fits the device; else the iteration graphs */
+  int64_t train_launches = 0;     /* of k_mlp_train */
 };
 
 namespace {
@@ -1290,6 +1291,7 @@ int mlp_train_cluster(SppMlp* m, int B, int iters, float lr) {
     a.bias = m->bias + done;
     a.iters = iters - done < most ? iters - done : most;
     MCUDA(cudaLaunchKernelEx(&cfg, k_mlp_train, a));
+    m->train_launches++;
   }
   return SPP_OK;
 }
@@ -1348,6 +1350,8 @@ int spp_mlp_destroy(SppMlp* m) {
   delete m;
   return SPP_OK;
 }
+
+int64_t spp_mlp_resident_launches(SppMlp* m) { return m ? m->train_launches : 0; }
 
 int spp_mlp_num_params(SppMlp* m) { return m ? m->P : 0; }
 

@@ -126,6 +126,10 @@ class Mlp:
                                          abi.fptr(g), abi.fptr(loss)), "spp_mlp_grad")
         return g, loss
 
+    def resident_launches(self):
+        """Launches so far that ran many training iterations each."""
+        return int(abi.lib().spp_mlp_resident_launches(self._h))
+
     def train(self, x, t, iters=2000, lr=1e-3, weights=None):
         x = np.ascontiguousarray(x, np.float32)
         t = np.ascontiguousarray(t, np.float32)

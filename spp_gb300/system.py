@@ -143,7 +143,12 @@ class System:
         return cx, cy
 
     def kernel_launches(self):
+        """Kernel passes run so far (a resident run counts those of its steps)."""
         return int(abi.lib().spp_kernel_launches(self._h))
+
+    def resident_launches(self):
+        """Resident runs launched so far (0: the system steps through graphs)."""
+        return int(abi.lib().spp_resident_launches(self._h))
 
     def stream(self):
         return abi.lib().spp_stream(self._h)
