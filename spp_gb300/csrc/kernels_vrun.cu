@@ -427,7 +427,8 @@ bool plan_vrun(const SppConsts& k, const DevState& d, VrunPlan* plan) {
    * places, flocks made most steps do so, 53 us per step against 26 with 32) */
   plan->cap = 32;
   while (plan->cap > 8 && cells * plan->cap * 2 * sizeof(float4) > (384ull << 20)) plan->cap /= 2;
-  return cells * plan->cap * 2 * sizeof(float4) <= (1ull << 30);
+  if (cells * plan->cap * 2 * sizeof(float4) > (1ull << 30)) plan->blocks = 0;   /* the general path */
+  return plan->blocks > 0;
 }
 
 int launch_vrun(const SppConsts& k, const DevState& d, const VrunPlan& plan, const VrunBufs& vb, int nsteps, int first,
