@@ -42,6 +42,7 @@
 #include "spp_internal.cuh"
 #include "spp_grid.cuh"
 #include "spp_pack.cuh"
+#include <algorithm>
 #include <type_traits>
 
 namespace {
@@ -421,13 +422,21 @@ bool plan_vrun(const SppConsts& k, const DevState& d, VrunPlan* plan) {
   plan->per_sm = per_sm;
   const uint64_t cells = ((uint64_t)d.D * d.D + 3) & ~3ull;
   plan->cells = (uint32_t)cells;
-  /* bucket places per cell: 32 while the two buffers stay within 384 MB, at
-   * least 8 (a unit cell at the usual densities holds a few particles; what
-   * does not fit goes through the sorted copy: at N = 97,281, eta = 0.3 and 16
-   * places, flocks made most steps do so, 53 us per step against 26 with 32) */
+  /* Bucket places per cell: 32, fewer (down to 4) where the cells are many for
+   * the particles, so that a dilute system does not hold memory by its area:
+   * at most 128 places per particle (density 1/4 with 32) or 2 million, and 12
+   * million at all (32 bytes each, 40 with the angle rule's headings: 384 and
+   * 480 MB); beyond that the general path (3,000 particles at L = 420 held 362
+   * MB of buckets, 10 MB now).  A unit cell at the usual densities holds a few
+   * particles; a step with a fuller cell goes through the sorted copy.  us per
+   * step with 32 / 16 / 8 / 4 places and of the general path, flocked (eta =
+   * 0.05, 3,000 steps on): N = 3,000 at density 0.1 5.0 / 5.0 / 10.8 / 11.1, 16.2;
+   * 50,000 at 0.25, angles, 14.3 / 19.7 / 20.4 / 20.2, 29.4; 175,000 at 0.1 43.3
+   * with any, 49.1. */
+  const uint64_t most = std::min<uint64_t>(12u << 20, std::max<uint64_t>(128u * (uint64_t)d.n, 2u << 20));
   plan->cap = 32;
-  while (plan->cap > 8 && cells * plan->cap * 2 * sizeof(float4) > (384ull << 20)) plan->cap /= 2;
-  if (cells * plan->cap * 2 * sizeof(float4) > (1ull << 30)) plan->blocks = 0;   /* the general path */
+  while (plan->cap > 4 && cells * plan->cap > most) plan->cap /= 2;
+  if (cells * plan->cap > most) plan->blocks = 0;
   return plan->blocks > 0;
 }
 
