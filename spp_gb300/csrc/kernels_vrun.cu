@@ -405,6 +405,14 @@ bool plan_vrun(const SppConsts& k, const DevState& d, VrunPlan* plan) {
   const int64_t total = (int64_t)d.n * lanes;
   if (total > room) return false;
   const int per_sm = total <= (int64_t)sms * vrun_threads(1) ? 1 : 2;
+  /* The push past one block per SM is taken too, although its step kernels,
+   * which have the registers, win in flocks: us per step resident / step
+   * kernels 200 steps in at eta = 0.3, density 1 (2; 1/2): N = 97,001 55 / 57 (85 / 91;
+   * 46 / 49), 100,001 65 / 61 (82 / 77; 52 / 50), 120,001 73 / 68 (114 / 102; 52 / 49),
+   * 175,001 89 / 82 (108 / 97; 63 / 60).  From a uniform start it is the other way
+   * round (upload, 10 steps, download: 120,001 370 / 446, with the first call's
+   * graph capture 415 / 630; 175,001 412 / 533, 466 / 712).  The other rules stay
+   * ahead in flocks as well (vector 27 / 31 at 175,001, angles 27 / 34). */
   int threads = (int)(((total + per_sm * sms - 1) / (per_sm * sms) + 31) / 32 * 32);
   if (threads < 128) threads = 128;
   const int blocks = (int)((total + threads - 1) / threads);
