@@ -24,8 +24,11 @@ namespace {
 
 thread_local std::string g_err;
 
+/* Reports a failure.  A CUDA call's error is taken off the thread with it:
+ * left there, the next call of any handle would meet it (cudaGetLastError) and
+ * fail in its turn. */
 int fail(int status, const std::string& msg) {
-  g_err = msg;
+  spp_internal_set_error(msg.c_str());
   return status;
 }
 
@@ -60,7 +63,10 @@ struct GraphEntry {
 
 }  // namespace
 
-void spp_internal_set_error(const char* msg) { g_err = msg ? msg : ""; }
+void spp_internal_set_error(const char* msg) {
+  g_err = msg ? msg : "";
+  cudaGetLastError();
+}
 
 struct SppSystem {
   SppParams p;
