@@ -238,7 +238,13 @@ int spp_upload_tumble(SppSystem* s, const int32_t* state, int n);
 /* Multi_Step(nsteps) (parallel/box.h:394-439): nsteps full integrator steps.
  * The neighbour list is rebuilt on device when a particle has moved more
  * than skin/2 since the last build.  Asynchronous on the handle's stream;
- * errors raised on the device are reported by the next spp_sync. */
+ * errors raised on the device are reported by the next spp_sync.
+ * On a stream that is being captured (spp_set_stream) the steps of a small
+ * Vicsek system are recorded: up to 16,384 particles and fewer than 65,536
+ * cells (side D = floor(2L / 1.001 r)) with 24 n + 8 D^2 <= 229,376 (20 n but for
+ * the angle rule).  A replay takes them again from where the system is;
+ * SppObservables.step follows.  Other systems are refused with SPP_ERR_CUDA, and
+ * the calls that wait cannot be captured. */
 int spp_step(SppSystem* s, int nsteps);
 /* Waits for the handle's stream and reports device-side status. */
 int spp_sync(SppSystem* s);

@@ -415,8 +415,13 @@ int get_graph(SppSystem* s, int nsteps, cudaGraphExec_t* out) {
   return SPP_OK;
 }
 
-/* Systems of up to 16,384 particles and fewer than 65,536 cells, with 24
- * bytes per particle and 8 per cell within 224 KB. */
+/* The systems that may be stepped on a stream that is being captured (spp_step
+ * in include/spp.h): of up to 16,384 particles and fewer than 65,536 cells,
+ * with 24 bytes per particle (20 but for the angle rule) and 8 per cell within
+ * 224 KB.  A rule of the interface, not of the resident kernel, which would run
+ * any: these always could (they fit one cluster's shared memory, once), the
+ * others were always refused, since a step graph can be neither captured nor
+ * launched there, and callers may rely on either. */
 bool vicsek_captures(const SppSystem* s) {
   const size_t n = (size_t)s->d.n, cells = (size_t)s->d.D * s->d.D;
   const size_t per_particle = s->p.model == SPP_MODEL_VICSEK_REF_ANGLE ? 24 : 20;
