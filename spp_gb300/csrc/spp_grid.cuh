@@ -9,7 +9,10 @@ namespace {
 
 /* polls of a barrier's counter before a block gives up (a poll takes about
  * 0.7 us: seconds; a barrier is normally met within microseconds) */
-constexpr int RUN_WAIT_LIMIT = 1 << 22;
+#ifndef SPP_RUN_WAIT_LIMIT
+#define SPP_RUN_WAIT_LIMIT (1 << 22)
+#endif
+constexpr int RUN_WAIT_LIMIT = SPP_RUN_WAIT_LIMIT;   /* 0: every wait gives up at once (a test's build) */
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
