@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
   constexpr bool ANGLE = MODEL == SPP_MODEL_VICSEK_REF_ANGLE;
   constexpr int NC = (9 + LANES - 1) / LANES;   /* cells per lane */
   constexpr int AT_ONCE = 3;                    /* cells whose loads are issued together */
-    constexpr int DEPTH = MODEL == SPP_MODEL_VICSEK ? 6 : 4;   /* candidates whose loads are issued together */
+  constexpr int DEPTH = MODEL == SPP_MODEL_VICSEK ? 6 : 4;   /* candidates whose loads are issued together */
   __shared__ unsigned s_word;
   __shared__ unsigned long long s_sum[2];
   const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31;

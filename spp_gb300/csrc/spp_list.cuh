@@ -53,12 +53,6 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
 constexpr int LIST_LOCAL = 16;
 constexpr int LIST_TRIP = 2;   /* candidates in flight */
 
-/* spp_list_order with the lane count known at compile time */
-template <int LANES>
-__device__ __forceinline__ uint32_t list_order(uint32_t id) {
-  return LANES == 1 ? id : ((id & 3u) << 30) | (id >> 2);
-}
-
 /* Batcher's odd-even merge sort (K. E. Batcher, Sorting networks and their
  * applications, 1968) of key[LO .. LO + N - 1]; entries from LIVE on hold the
  * largest key throughout, so comparisons with them are left out. */
