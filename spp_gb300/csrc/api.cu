@@ -196,15 +196,19 @@ void alloc_vrun(SppSystem* s) {
   b.cap = s->vrun.cap;
   Arena arena;
   for (int c = 0; c < 3; ++c) arena.want(&b.count[c], cells);
-  arena.want(&b.full, 3);
+  arena.want(&b.full, 5);
   for (int c = 0; c < 2; ++c) {
     arena.want(&b.bucket[c], places);
     if (s->p.model == SPP_MODEL_VICSEK_REF_ANGLE) arena.want(&b.bucket_th[c], places);
   }
-  if (arena.take(&s->vblock) != SPP_OK) {
+  /* all ones: dirty, and some phase */
+  if (arena.take(&s->vblock) != SPP_OK || cudaMemsetAsync(b.full, 1, 5 * sizeof(uint32_t), s->stream) != cudaSuccess) {
     cudaGetLastError();
     free_vrun(s);
+    return;
   }
+  b.dirty = b.full + 3;
+  b.phase = b.full + 4;
 }
 
 void free_dev(SppSystem* s) {

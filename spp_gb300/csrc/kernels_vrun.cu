@@ -79,7 +79,14 @@ __device__ __forceinline__ void vrun_pair(const SppConsts& k, VrunAcc* acc, floa
 /* Counts are kept for three steps, buckets for two: step t reads count
  * t % 3 and bucket t % 2, fills (t + 1) % 3 and (t + 1) % 2, and clears count
  * (t + 2) % 3, which every block has finished reading before the barrier of
- * step t - 1.  full[c]: some cell of count c overflowed its bucket. */
+ * step t - 1.  full[c]: some cell of count c overflowed its bucket.
+ * The last step fills nothing, so a launch leaves two clean counts, and the
+ * next goes on with them (t % 3 stands for (t + *vb.phase) % 3): it clears the
+ * third in its first step, and the one barrier after the particles are in
+ * their cells is all that it pays to start.  us per call of one step, counts
+ * cleared behind a barrier at the start and one more barrier at the end / now:
+ * vector rule N = 1 10.5 / 8.7, 300 10.8 / 8.7, 4,096 14.0 / 10.8, 50,001 22.8 / 18.0
+ * (one cluster of 16 CTAs took 8.7, 10.7 and 17.9 for the first three). */
 template <int MODEL, int LANES, int PER_SM>
 __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
     k_vrun(const __grid_constant__ SppConsts k, const __grid_constant__ DevState d, const __grid_constant__ VrunBufs vb,
@@ -99,6 +106,12 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
   const bool inb = i < n;
   const bool head = inb && lane_r == 0;
   if (ctl->run_timeout) return;   /* the same for every block */
+  const bool dirty = *vb.dirty != 0u;
+  /* counts and flags of the step at hand, of the next, and those to be cleared
+   * (in registers, rotated: indices cost the angle rule 3%) */
+  const uint32_t phase = *vb.phase % 3u;
+  uint32_t *cnow = vb.count[phase], *cnext = vb.count[(phase + 1u) % 3u], *cold = vb.count[(phase + 2u) % 3u];
+  uint32_t *fnow = vb.full + phase, *fnext = vb.full + (phase + 1u) % 3u, *fold = vb.full + (phase + 2u) % 3u;
   uint32_t step = ctl->step, sorted = ctl->run_sorted;
   unsigned target = 0;
   auto barrier = [&]() -> bool {
@@ -107,6 +120,7 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
     if (tid == 0) {
       grid_arrive(ctl);
       s_word = grid_wait(ctl, target);
+      if (s_word == 0u) *vb.dirty = 1u;
     }
     __syncthreads();
     return s_word != 0u;
@@ -123,18 +137,18 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
   int cx = 0, cy = 0;
   uint32_t rank = 0u;
   /* the particle's place among the cells of step t */
-  auto insert = [&](int t) {
+  auto insert = [&](int t, uint32_t* counts, uint32_t* flag) {
     if (head) {
       cx = spp_cell_coord(p.x, k.L, k.L2, D, SPP_BIN_GEOMETRIC);
       cy = spp_cell_coord(p.y, k.L, k.L2, D, SPP_BIN_GEOMETRIC);
       const uint32_t cell = (uint32_t)cy * (uint32_t)D + (uint32_t)cx;
-      rank = atomicAdd(vb.count[t % 3] + cell, 1u);
+      rank = atomicAdd(counts + cell, 1u);
       if (rank < (uint32_t)K) {
         const size_t at = (size_t)cell * K + rank;
         vb.bucket[t & 1][at] = make_float4(p.x, p.y, pack_fx(p.z), pack_fx(p.w));
         if (ANGLE) vb.bucket_th[t & 1][at] = th;
       } else {
-        vb.full[t % 3] = 1u;
+        *flag = 1u;
       }
     }
     if (LANES > 1) {
@@ -146,23 +160,46 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
       rank = __shfl_sync(0xffffffffu, rank, src);
     }
   };
+  /* the block's part of the heading sums of k_polarization: exact, whatever
+   * the order */
+  auto frame_sums = [&]() {
+    long long sx = 0, sy = 0;
+    if (head) {
+      spp_fx hx = {0, 0}, hy = {0, 0};
+      spp_fx_add(&hx, p.z);
+      spp_fx_add(&hy, p.w);
+      sx = spp_fx_units(hx);
+      sy = spp_fx_units(hy);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sx += __shfl_down_sync(0xffffffffu, sx, o);
+      sy += __shfl_down_sync(0xffffffffu, sy, o);
+    }
+    if (lane == 0) {
+      atomicAdd(&s_sum[0], (unsigned long long)sx);
+      atomicAdd(&s_sum[1], (unsigned long long)sy);
+    }
+  };
   if (tid < 2) s_sum[tid] = 0ull;
-  for (uint32_t c = gtid; c < vb.cells; c += gthreads) vb.count[0][c] = vb.count[1][c] = vb.count[2][c] = 0u;
-  if (gtid < 3) vb.full[gtid] = 0u;
-  if (!barrier()) return;
-  insert(0);
+  if (dirty) {   /* the same for every block: written behind a barrier or by an earlier launch */
+    for (uint32_t c = gtid; c < vb.cells; c += gthreads) vb.count[0][c] = vb.count[1][c] = vb.count[2][c] = 0u;
+    if (gtid < 3) vb.full[gtid] = 0u;
+    if (!barrier()) return;
+    if (gtid == 0) *vb.dirty = 0u;
+  }
+  insert(0, cnow, fnow);
   uint32_t word = head ? spp_draw_k(&k, pid, step, SPP_RNG_VICSEK).v[0] : 0u;
   if (!barrier()) return;
 
   int to_frame = first;
-  for (int t = 0; t < nsteps; ++t, ++step) {
+  for (int t = 0;; ++t, ++step) {
     {
-      uint32_t* const clear = vb.count[(t + 2) % 3];
-      for (uint32_t c = gtid; c < vb.cells; c += gthreads) clear[c] = 0u;
-      if (gtid == 0) vb.full[(t + 2) % 3] = 0u;
+      for (uint32_t c = gtid; c < vb.cells; c += gthreads) cold[c] = 0u;
+      if (gtid == 0) *fold = 0u;
     }
-    const uint32_t* const count = vb.count[t % 3];
-    const unsigned full = *(volatile const unsigned*)(vb.full + t % 3);   /* the same for every thread of the grid */
+    const uint32_t* const count = cnow;
+    const unsigned full = *(volatile const unsigned*)fnow;   /* the same for every thread of the grid */
     if (full || spp_sort_due(step, sorted)) {
       sorted = step;
       /* the particles change hands in cell order, so that a warp's threads
@@ -304,28 +341,20 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
         d.img[i] = make_int2(g.x + gx, g.y + gy);
       }
     }
-    insert(t + 1);
     const bool frame = every > 0 && --to_frame == 0;
-    if (frame) {
-      /* the heading sums of k_polarization: exact, whatever the order */
-      long long sx = 0, sy = 0;
-      if (head) {
-        spp_fx hx = {0, 0}, hy = {0, 0};
-        spp_fx_add(&hx, p.z);
-        spp_fx_add(&hy, p.w);
-        sx = spp_fx_units(hx);
-        sy = spp_fx_units(hy);
+    if (t + 1 == nsteps) {   /* nothing of this launch follows */
+      if (frame) {
+        frame_sums();
+        __syncthreads();
+        if (tid == 0) {
+          atomicAdd(sums, s_sum[0]);
+          atomicAdd(sums + 1, s_sum[1]);
+        }
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        sx += __shfl_down_sync(0xffffffffu, sx, o);
-        sy += __shfl_down_sync(0xffffffffu, sy, o);
-      }
-      if (lane == 0) {
-        atomicAdd(&s_sum[0], (unsigned long long)sx);
-        atomicAdd(&s_sum[1], (unsigned long long)sy);
-      }
+      break;
     }
+    insert(t + 1, cnext, fnext);
+    if (frame) frame_sums();
     target += gridDim.x;
     __syncthreads();
     if (tid == 0) {
@@ -340,9 +369,22 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
       sums += 2;
       to_frame = every;
     }
+    {
+      uint32_t* const c = cnow;
+      cnow = cnext;
+      cnext = cold;
+      cold = c;
+      uint32_t* const f = fnow;
+      fnow = fnext;
+      fnext = fold;
+      fold = f;
+    }
     /* the next step's noise while the other blocks arrive */
     if (head) word = spp_draw_k(&k, pid, step + 1u, SPP_RNG_VICSEK).v[0];
-    if (tid == 0) s_word = grid_wait(ctl, target);
+    if (tid == 0) {
+      s_word = grid_wait(ctl, target);
+      if (s_word == 0u) *vb.dirty = 1u;
+    }
     __syncthreads();
     if (s_word == 0u) return;
   }
@@ -354,8 +396,9 @@ __global__ void __launch_bounds__(vrun_threads(PER_SM), PER_SM)
   }
   if (tid == 0) {
     if (blockIdx.x == 0) {
-      ctl->step = step;
+      ctl->step = step + 1u;
       ctl->run_sorted = sorted;
+      *vb.phase = (phase + (uint32_t)nsteps) % 3u;
       ctl->need_rebuild = 0u;
     }
     /* the last block to leave clears the barrier for the next launch */

@@ -178,7 +178,9 @@ struct VrunPlan {
 };
 struct VrunBufs {
   uint32_t* count[3];
-  uint32_t* full;         /* [3] */
+  uint32_t* full;         /* [3], then the two words that a launch leaves to the next: */
+  uint32_t* dirty;        /* not 0: counts and full are to be cleared first (new buffers, a barrier that gave up) */
+  uint32_t* phase;        /* which of the counts the next launch starts with */
   float4* bucket[2];      /* [cells][cap] */
   float* bucket_th[2];    /* headings, angle rule only */
   uint32_t cells;
