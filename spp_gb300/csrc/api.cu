@@ -767,6 +767,19 @@ int spp_internal_mark(SppSystem* s, double2** xy, float** th, int64_t** step) {
   return SPP_OK;
 }
 
+int spp_internal_scratch(SppSystem* s, size_t words, unsigned long long** out) {
+  if (words > s->obs_nbins) {
+    if (s->obs_bins) cudaFree(s->obs_bins);
+    s->obs_bins = nullptr;
+    s->obs_nbins = 0;
+    int rc = dalloc(&s->obs_bins, words);
+    if (rc != SPP_OK) return rc;
+    s->obs_nbins = words;
+  }
+  *out = s->obs_bins;
+  return SPP_OK;
+}
+
 int spp_internal_obs_space(SppSystem* s, size_t cells, size_t bins, uint32_t** count, uint32_t** start, uint32_t** tmp,
                            unsigned long long** counts) {
   if (cells > s->d.n_keys && cells > s->obs_cells) {
@@ -778,19 +791,12 @@ int spp_internal_obs_space(SppSystem* s, size_t cells, size_t bins, uint32_t** c
     if (rc != SPP_OK) return rc;
     s->obs_cells = padded;
   }
-  if (bins > s->obs_nbins) {
-    if (s->obs_bins) cudaFree(s->obs_bins);
-    s->obs_bins = nullptr;
-    s->obs_nbins = 0;
-    int rc = dalloc(&s->obs_bins, bins);
-    if (rc != SPP_OK) return rc;
-    s->obs_nbins = bins;
-  }
+  int rc = spp_internal_scratch(s, bins, counts);
+  if (rc != SPP_OK) return rc;
   const bool own = cells > s->d.n_keys;
   *count = own ? s->obs_grid : s->d.cell_count;
   *start = own ? s->obs_grid + s->obs_cells : s->d.cell_start;
   *tmp = own ? s->obs_grid + 2 * s->obs_cells : s->d.scan_tmp;
-  *counts = s->obs_bins;
   return SPP_OK;
 }
 

@@ -379,6 +379,26 @@ void shape_from_sums(const double* m, int n, double* cm_x, double* cm_y, double*
   *delta = dl * dl;
 }
 
+/* Device words of one call: the system's scratch, kept, or memory of their own
+ * where they are many (a series of more than half a million frames).  An
+ * allocation of a few words per call costs 130 us next to a large system, whose
+ * own arrays are one allocation: the few words take, and give back, a page of
+ * device memory (series of 5 frames, us: 60,001 disks 346 -> 211, 400,001 552 ->
+ * 412, 1M 894 -> 748). */
+struct CallWords {
+  unsigned long long* p = nullptr;
+  bool own = false;
+  ~CallWords() {
+    if (own) cudaFree(p);
+  }
+  int take(SppSystem* s, size_t n) {
+    if (n <= (1u << 20)) return spp_internal_scratch(s, n, &p);
+    if (cudaMalloc((void**)&p, sizeof(*p) * n) != cudaSuccess) return ofail(SPP_ERR_ALLOC, "cudaMalloc failed");
+    own = true;
+    return SPP_OK;
+  }
+};
+
 inline int nblk(int n) { return (n + SPP_BLOCK - 1) / SPP_BLOCK; }
 
 int hist_edges(bool radial, const HistArgs& h) { return radial ? h.nbins + 1 : h.gx + h.gy + 2; }
@@ -526,8 +546,10 @@ int spp_polarization_series(SppSystem* s, int nframes, int every, double* p, dou
   cudaStream_t st;
   int rc = spp_internal_view(s, &d, &k, &st);
   if (rc != SPP_OK) return rc;
-  unsigned long long* sums = nullptr;
-  OCUDA(cudaMalloc((void**)&sums, sizeof(unsigned long long) * 2 * (size_t)nframes));
+  CallWords words;
+  rc = words.take(s, 2 * (size_t)nframes);
+  if (rc != SPP_OK) return rc;
+  unsigned long long* const sums = words.p;
   std::vector<long long> host(2 * (size_t)nframes);
   cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(unsigned long long) * 2 * (size_t)nframes, st);
   /* the Verlet-list models may freeze on a full neighbour list; their frames
@@ -553,7 +575,6 @@ int spp_polarization_series(SppSystem* s, int nframes, int every, double* p, dou
     e = cudaMemcpyAsync(host.data(), sums, sizeof(long long) * host.size(), cudaMemcpyDeviceToHost, st);
   if (rc == SPP_OK && e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (rc == SPP_OK && e == cudaSuccess && !listed) rc = spp_sync(s);   /* device-side status */
-  cudaFree(sums);
   if (rc != SPP_OK) return rc;
   if (e != cudaSuccess) return ofail(SPP_ERR_CUDA, cudaGetErrorString(e));
   const double inv = 1.0 / 134217728.0; /* fixed-point units of 2^-27 */
@@ -616,15 +637,16 @@ int spp_ring_shapes(SppSystem* s, SppRingShape* out, int n_rings) {
   const int nr = k.n_beads / k.ring_size;
   if (n_rings != nr) return ofail(SPP_ERR_INVALID, "n_rings differs from the system's ring count");
   const int sw = (d.n - k.n_beads) / nr;
-  double* sums = nullptr;
-  OCUDA(cudaMalloc((void**)&sums, sizeof(double) * 10 * (size_t)nr));
+  CallWords words;
+  rc = words.take(s, 10 * (size_t)nr);
+  if (rc != SPP_OK) return rc;
+  double* const sums = reinterpret_cast<double*>(words.p);
   k_obs_ring_sums<<<2 * nr, SPP_BLOCK, 0, st>>>(d, k, nr, k.ring_size, sw, sums);
   spp_internal_count_launches(s, 1);
   std::vector<double> h(10 * (size_t)nr);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), sums, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(sums);
   if (e != cudaSuccess) return ofail(SPP_ERR_CUDA, std::string("ring shapes: ") + cudaGetErrorString(e));
   for (int r = 0; r < nr; ++r) {
     SppRingShape& o = out[r];
@@ -685,15 +707,16 @@ int spp_ring_motion(SppSystem* s, SppRingMotion* out, int n_rings) {
   if (now <= *mark) return ofail(SPP_ERR_INVALID, "no step taken since the marked frame");
   const double elapsed = (double)(now - *mark) * spp_internal_dt(s);
   const int sw = (d.n - k.n_beads) / nr;
-  double* sums = nullptr;
-  OCUDA(cudaMalloc((void**)&sums, sizeof(double) * 2 * MOTION_SUMS * (size_t)nr));
+  CallWords words;
+  rc = words.take(s, 2 * MOTION_SUMS * (size_t)nr);
+  if (rc != SPP_OK) return rc;
+  double* const sums = reinterpret_cast<double*>(words.p);
   k_obs_ring_motion<<<2 * nr, SPP_BLOCK, 0, st>>>(d, k, nr, k.ring_size, sw, xy, th, 1.0 / elapsed, sums);
   spp_internal_count_launches(s, 1);
   std::vector<double> h(2 * MOTION_SUMS * (size_t)nr);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), sums, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(sums);
   if (e != cudaSuccess) return ofail(SPP_ERR_CUDA, std::string("ring motion: ") + cudaGetErrorString(e));
   for (int r = 0; r < nr; ++r) {
     /* Compute_All_Variables, parallel/beadbox.h:385-428 */

@@ -116,6 +116,8 @@ int spp_internal_mark(SppSystem* s, double2** xy, float** th, int64_t** step);
  * arrays where they are large enough), and `bins` 64-bit counts */
 int spp_internal_obs_space(SppSystem* s, size_t cells, size_t bins, uint32_t** count, uint32_t** start, uint32_t** tmp,
                            unsigned long long** counts);
+/* api.cu: `words` 64-bit words of the same scratch, for one call's sums */
+int spp_internal_scratch(SppSystem* s, size_t words, unsigned long long** out);
 /* api.cu: nframes x every steps of a resident Vicsek run with the heading
  * sums of every frame; 1: not such a system, < 0: error (message set) */
 int spp_internal_series(SppSystem* s, int nframes, int every, unsigned long long* sums);
