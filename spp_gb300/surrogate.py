@@ -276,7 +276,7 @@ def run_sweep(points, max_steps=20000, window=500, pilot_frac=0.2, holdout_frac=
     before any exist, on the held-out points or, with first_scale="oof",
     the out-of-fold multiplier).  Measured on the 512-point workload (one
     GB300, points/hour at |dP| <= 0.02 against the plain batched sweep, with
-    batch kernels that took 16.8 s for it, now 10.4), coverage 0.9: held-out first scale with one round 1.07x, with two rounds
+    batch kernels that took 16.8 s for it, now 10.0), coverage 0.9: held-out first scale with one round 1.07x, with two rounds
     1.01x; out-of-fold first scale with two rounds 1.03x.  The coverage
     trades retirements for accuracy (held-out first scale, one round):
     0.9 -> 1.07x, 98.3% of the retired points within tolerance; 0.8 (the
