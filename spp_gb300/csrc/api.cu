@@ -104,7 +104,6 @@ struct SppSystem {
   bool use_graphs = true;
   VrunPlan vrun = {0, 0, 0, 0, 0, 0};   /* the same for the Vicsek models (k_vrun) */
   VrunBufs vbuf = {};
-  char* vblock = nullptr;
   RunPlan run = {0, 0, 0};          /* resident runs (k_run): launch shape, 0 blocks = the step graphs */
   /* staging for uploads/downloads: x, y, theta, then the x and y counters
    * (int32), n entries each, in one device allocation */
@@ -112,7 +111,7 @@ struct SppSystem {
   float* stage_y = nullptr;
   float* stage_t = nullptr;
   int32_t* stage_img = nullptr;
-  char* block = nullptr;         /* every device array of d but the list, and stage_* */
+  char* block = nullptr;         /* every device array of d but the list, stage_* and vbuf's */
   HostBlock* host = nullptr;     /* pinned: what a call reads back with one wait */
   std::vector<GraphEntry> graphs;
   /* tangent-space (Lyapunov) estimator */
@@ -179,36 +178,19 @@ void free_lyap(SppSystem* s) {
   s->lyap_on = false;
 }
 
-void free_vrun(SppSystem* s) {
-  if (s->vblock) cudaFree(s->vblock);
-  s->vblock = nullptr;
-  s->vbuf = {};
-  s->vrun.blocks = 0;
-}
-
-/* The cell buckets of a resident Vicsek run.  Without the memory the system
- * steps through the launches of the general path. */
-void alloc_vrun(SppSystem* s) {
+/* The cell buckets of a resident Vicsek run. */
+void want_vrun(SppSystem* s, Arena* arena) {
   VrunBufs& b = s->vbuf;
   const size_t cells = s->vrun.cells, places = cells * s->vrun.cap;
   b = {};
   b.cells = s->vrun.cells;
   b.cap = s->vrun.cap;
-  Arena arena;
-  for (int c = 0; c < 3; ++c) arena.want(&b.count[c], cells);
-  arena.want(&b.full, 5);
+  for (int c = 0; c < 3; ++c) arena->want(&b.count[c], cells);
+  arena->want(&b.full, 5);
   for (int c = 0; c < 2; ++c) {
-    arena.want(&b.bucket[c], places);
-    if (s->p.model == SPP_MODEL_VICSEK_REF_ANGLE) arena.want(&b.bucket_th[c], places);
+    arena->want(&b.bucket[c], places);
+    if (s->p.model == SPP_MODEL_VICSEK_REF_ANGLE) arena->want(&b.bucket_th[c], places);
   }
-  /* all ones: dirty, and some phase */
-  if (arena.take(&s->vblock) != SPP_OK || cudaMemsetAsync(b.full, 1, 5 * sizeof(uint32_t), s->stream) != cudaSuccess) {
-    cudaGetLastError();
-    free_vrun(s);
-    return;
-  }
-  b.dirty = b.full + 3;
-  b.phase = b.full + 4;
 }
 
 void free_dev(SppSystem* s) {
@@ -230,7 +212,8 @@ void free_dev(SppSystem* s) {
   s->stage_img = nullptr;
   if (s->host) cudaFreeHost(s->host);
   s->host = nullptr;
-  free_vrun(s);
+  s->vbuf = {};
+  s->vrun.blocks = 0;
 }
 
 double interaction_radius(const SppParams& p) { return spp_interaction_range(&p); }
@@ -939,35 +922,57 @@ int spp_create(const SppParams* p, SppSystem** out) {
     delete s;
     return fail(SPP_ERR_INVALID, "cell grid too large for the scan");
   }
-  Arena arena;
-  arena.want(&d.pos, n);
-  arena.want(&d.half, s->uses_list ? n : 1);
-  arena.want(&d.half2, s->nstages > 2 ? n : 1);
-  arena.want(&d.theta, n);
-  arena.want(&d.img, n);
-  arena.want(&d.id, n);
-  if (p->model == SPP_MODEL_BEADS) arena.want(&d.inv, n);
-  if (s->k.tumble) arena.want(&d.tumble, n);
-  arena.want(&d.kacc, s->nstages > 2 ? n : 1);
-  arena.want(&d.dth, s->nstages > 1 ? n : 1);
-  arena.want(&d.ref, n);
-  arena.want(&d.pos_alt, n);
-  arena.want(&d.theta_alt, n);
-  arena.want(&d.img_alt, n);
-  arena.want(&d.id_alt, n);
-  arena.want(&d.key, n);
-  arena.want(&d.rank, n);
-  arena.want(&d.cell_count, d.n_keys);
-  arena.want(&d.cell_start, d.n_keys);
-  arena.want(&d.scan_tmp, nscan);
-  arena.want(&d.nn, n);
-  arena.want(&d.long_q, n);
-  if (s->k.lanes > 1) arena.want(&d.nn_lanes, n);
-  arena.want(&d.ctl, 1);
-  arena.want(&d.red, 4);
-  arena.want(&d.run_sums, RUN_MAX_BLOCKS);
-  arena.want(&s->stage_x, 5 * n);
-  rc = arena.take(&s->block);
+  {
+    const char* rv = getenv("SPP_RESIDENT");
+    const char* sv = getenv("SPP_VICSEK_SMALL");
+    const bool off = rv && rv[0] == '0';
+    if (s->uses_list && !off) plan_run(s->k, d, &s->run);
+    if (!s->uses_list && !off && !(sv && sv[0] == '0')) plan_vrun(s->k, d, &s->vrun);
+  }
+  auto lay_out = [&](Arena* arena) {
+    arena->want(&d.pos, n);
+    arena->want(&d.half, s->uses_list ? n : 1);
+    arena->want(&d.half2, s->nstages > 2 ? n : 1);
+    arena->want(&d.theta, n);
+    arena->want(&d.img, n);
+    arena->want(&d.id, n);
+    if (p->model == SPP_MODEL_BEADS) arena->want(&d.inv, n);
+    if (s->k.tumble) arena->want(&d.tumble, n);
+    arena->want(&d.kacc, s->nstages > 2 ? n : 1);
+    arena->want(&d.dth, s->nstages > 1 ? n : 1);
+    arena->want(&d.ref, n);
+    arena->want(&d.pos_alt, n);
+    arena->want(&d.theta_alt, n);
+    arena->want(&d.img_alt, n);
+    arena->want(&d.id_alt, n);
+    arena->want(&d.key, n);
+    arena->want(&d.rank, n);
+    arena->want(&d.cell_count, d.n_keys);
+    arena->want(&d.cell_start, d.n_keys);
+    arena->want(&d.scan_tmp, nscan);
+    arena->want(&d.nn, n);
+    arena->want(&d.long_q, n);
+    if (s->k.lanes > 1) arena->want(&d.nn_lanes, n);
+    arena->want(&d.ctl, 1);
+    arena->want(&d.red, 4);
+    arena->want(&d.run_sums, RUN_MAX_BLOCKS);
+    arena->want(&s->stage_x, 5 * n);
+    if (s->vrun.blocks > 0) want_vrun(s, arena);
+  };
+  {
+    Arena arena;
+    lay_out(&arena);
+    rc = arena.take(&s->block);
+  }
+  if (rc != SPP_OK && s->vrun.blocks > 0) {
+    /* without the memory for the buckets the system steps through the launches
+     * of the general path */
+    s->vrun.blocks = 0;
+    s->vbuf = {};
+    Arena arena;
+    lay_out(&arena);
+    rc = arena.take(&s->block);
+  }
   if (rc == SPP_OK) {
     s->stage_y = s->stage_x + n;
     s->stage_t = s->stage_x + 2 * n;
@@ -987,19 +992,18 @@ int spp_create(const SppParams* p, SppSystem** out) {
   cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMemsetAsync(d.ctl, 0, sizeof(Ctl), s->stream);
+  if (e == cudaSuccess && s->vrun.blocks > 0) {
+    VrunBufs& b = s->vbuf;
+    b.dirty = b.full + 3;
+    b.phase = b.full + 4;
+    e = cudaMemsetAsync(b.full, 1, 5 * sizeof(uint32_t), s->stream);   /* all ones: dirty, and some phase */
+  }
   if (e != cudaSuccess) {
     free_dev(s);
     delete s;
     return fail(SPP_ERR_CUDA, std::string("stream/ctl setup: ") + cudaGetErrorString(e));
   }
   s->own_stream = true;
-  {
-    const char* rv = getenv("SPP_RESIDENT");
-    const char* sv = getenv("SPP_VICSEK_SMALL");
-    const bool off = rv && rv[0] == '0';
-    if (s->uses_list && !off) plan_run(s->k, d, &s->run);
-    if (!s->uses_list && !off && !(sv && sv[0] == '0') && plan_vrun(s->k, d, &s->vrun)) alloc_vrun(s);
-  }
   s->per_rebuild_kernels = 6;   /* bin_count, scan x2, scatter, build_list, sort_long */
   s->per_step_kernels = s->uses_list ? (s->nstages == 1 ? 2 : s->nstages) : 5;
   *out = s;
