@@ -64,10 +64,9 @@ int g_na_next = 0;   /* slot replaced next once the table is full */
 typedef CUresult(CUDAAPI* NaCtxGetCurrent)(CUcontext*);
 typedef CUresult(CUDAAPI* NaCtxGetId)(CUcontext, unsigned long long*);
 
-/* Unique id of the calling thread's current context; false if there is none
- * (the runtime has not made one current on this thread yet) or the driver
- * does not offer the entry points. */
-bool na_current_context(unsigned long long* id) {
+}  // namespace
+
+bool spp_internal_context(unsigned long long* id) {
   static std::once_flag once;
   static NaCtxGetCurrent get_current = nullptr;
   static NaCtxGetId get_id = nullptr;
@@ -88,6 +87,8 @@ bool na_current_context(unsigned long long* id) {
   if (get_current(&c) != CUDA_SUCCESS || !c) return false;
   return get_id(c, id) == CUDA_SUCCESS;
 }
+
+namespace {
 
 NaScratch* na_lookup(unsigned long long id) {
   std::lock_guard<std::mutex> g(g_na_mu);
@@ -243,7 +244,7 @@ extern "C" int spp_pairs_noalloc(const float* x, const float* y, int n, double L
    * code, which a stream capture must not see: inside a capture only an
    * address found earlier in the same context is used. */
   unsigned long long ctx = 0;
-  bool have_ctx = na_current_context(&ctx);
+  bool have_ctx = spp_internal_context(&ctx);
   NaScratch* s = have_ctx ? na_lookup(ctx) : nullptr;
   cudaError_t e;
   if (!s) {
@@ -260,7 +261,7 @@ extern "C" int spp_pairs_noalloc(const float* x, const float* y, int n, double L
     if (e != cudaSuccess)
       return na_fail(SPP_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
     s = reinterpret_cast<NaScratch*>(p);
-    if (!have_ctx) have_ctx = na_current_context(&ctx);
+    if (!have_ctx) have_ctx = spp_internal_context(&ctx);
     if (have_ctx) na_remember(ctx, s);
   }
   int bits = 0;

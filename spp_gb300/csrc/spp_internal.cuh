@@ -121,6 +121,10 @@ int spp_internal_scratch(SppSystem* s, size_t words, unsigned long long** out);
 /* api.cu: nframes x every steps of a resident Vicsek run with the heading
  * sums of every frame; 1: not such a system, < 0: error (message set) */
 int spp_internal_series(SppSystem* s, int nframes, int every, unsigned long long* sums);
+/* noalloc.cu: unique id of the calling thread's current context; false if
+ * there is none (the runtime has not made one current on this thread yet) or
+ * the driver does not offer the entry points */
+bool spp_internal_context(unsigned long long* id);
 /* api.cu: the absolute step counter (waits for the stream); -1 on error */
 int64_t spp_internal_step(SppSystem* s);
 /* api.cu: the time step as given (double) */
