@@ -58,9 +58,10 @@ size_t host_block_bytes(int n) { return sizeof(HostBlock) + (n <= HOST_FRAME ? 5
 
 /* Pinned memory costs 100 us to get and 150 to give back, a fifth each of a
  * short life of a small system (create, upload, 5 steps, two downloads, destroy:
- * 64 Vicsek particles 668 -> 359 us, 16,384 disks 952 -> 644).  Blocks of
- * destroyed systems are kept for the next: sizes are powers of two from 4 KB,
- * at most HOST_SPARES blocks and HOST_SPARE_BYTES in all, by context (ids are
+ * 64 Vicsek particles 668 -> 337 us, 16,384 disks 952 -> 622).  Blocks of
+ * destroyed systems are kept for the next: whole pages, rounded up by less than
+ * a quarter so that systems of about the same size share them, at most
+ * HOST_SPARES blocks and HOST_SPARE_BYTES in all, by context (ids are
  * never used twice, so a block of a context that was reset is not taken
  * again). */
 constexpr int HOST_SPARES = 64;
@@ -76,9 +77,10 @@ int g_spares = 0;
 size_t g_spare_bytes = 0;
 
 size_t host_block_size(int n) {
-  size_t size = 4096;
-  while (size < host_block_bytes(n)) size *= 2;
-  return size;
+  const size_t want = (host_block_bytes(n) + 4095) / 4096 * 4096;
+  size_t step = 4096;
+  while (8 * step < want) step *= 2;
+  return (want + step - 1) / step * step;
 }
 
 /* *context: the current one, 0 if not known. */
